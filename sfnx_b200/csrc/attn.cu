@@ -107,36 +107,70 @@ __global__ void k_attn_prep_append(float* qg, float* k, const float* v, const fl
 // The reference's statement (src/kernels.cu:497-606) fixes, for every (row, head), a split of the row's owned positions
 // into 16 runs of `len` rows, chunks of 32 positions inside a run, a score as one fused chain over the head dimension,
 // an online-softmax step per chunk (warp xor-trees over the chunk's 32 weights) and value rows added in ascending
-// position; this kernel keeps all of that and changes who does it.  One block takes (run s, KV head, group of rows):
-// the rows of a window that read the same K/V (the same sequence) and have the same `len` walk the same chunks, so the
-// block stages each chunk of K and V once, as f32, and applies it to every (row, head) pair of the group - up to 96
-// pairs at a time - instead of once per row.  Rows group themselves on the device: block z = t works only if row t is
-// the first of its group, and then takes every later row of the group with it.
-//   scores : warp w holds pairs w, w + 8, ...; lane = position of the chunk; 12 independent chains a thread, the
-//            pair's query row read as float4 broadcasts
-//   softmax: the pair's 32 weights sit across the lanes of one warp, as the reference's trees want them
-//   values : thread = head dimension, one accumulator per pair in registers, the chunk's 32 V values of that
-//            dimension in registers too
-// PT is how many (row, head) pairs a block applies a chunk to at a time: 96 for the groups of rows that attend every owned
-// position, 8 or 16 (a pair or two a warp, more blocks an SM) for a row with a list of its own, which shares its chunks
-// with no other row.
+// position; this kernel keeps all of that and changes who does it.  A block takes (run s, KV head, PT of a group's (row,
+// head) pairs): the rows of a window that read the same K/V (the same sequence) and have the same `len` walk the same
+// chunks, so a block stages TILE positions of K once and applies them to all of its pairs.  Rows group themselves on the
+// device: row t leads a group if no earlier row belongs to it, and the blocks of a row that leads none leave.
+//   scores : lane = position (two a lane), a warp QW pairs: K is read from shared memory as stored (a step over eight
+//            dimensions: 4 wavefronts a position for all of the warp's pairs) and unpacked in registers, the queries as
+//            broadcasts of one wavefront; a chain a (position, pair), the chains of a step interleaved;
+//   softmax: the pair's 32 weights sit across the lanes of one warp, as the reference's trees want them; the weights
+//            replace the scores in shared memory;
+//   values : a thread holds VD dimensions x VP pairs of accumulators and walks the positions in ascending order.
+// K of the next tile is copied (cp.async) while the values of this one are added, V of this tile while its scores are
+// taken; a narrow block (every V value is one thread's) asks for a tile's V values straight into registers instead.
+// What bounds it is the fused steps (T heads ctx 512 of them): with 16-byte reads that hand the same K words to several
+// groups of lanes (a thread tile of 2 or 4 positions x 3 pairs) the shared-memory pipe was the limit, since a 16-byte read
+// costs four wavefronts however many of its words coincide.
+// Measured (one layer, 24 / 4 heads of 256): 16 rows over 32 768 positions 3360 -> 520 us (f16 rows), 3290 -> 590 (int8);
+// two rows each of six sequences of 14 336 positions 2660 -> 245, where a tile of 96 pairs held 12.
+// PT 48 in blocks of 256 threads for the rows of one sequence, PT 12 in blocks of 128, three an SM, where a group is
+// one or two rows: rows of several sequences, rows with a list, windows of one or two rows.
 // scratch: acc [T][nq][16][hd], then (m, z) [T][nq][16].
 struct AttPart {
     float m, z;
 };
-constexpr int AX_THREADS = 256, AX_WARPS = AX_THREADS / 32, AX_PT = 96, AX_PPW = AX_PT / AX_WARPS;
+constexpr int AX_THREADS = 256, AX_WARPS = AX_THREADS / 32;   // (k_attn_cells)
+template <int PT> struct AxShape {
+    static constexpr int THREADS = PT == 48 ? 256 : 128, TILE = PT == 48 ? 128 : 64, QW = PT == 48 ? 12 : 3, VD = PT == 48 ? 4 : 2, BLOCKS = PT == 48 ? 1 : 3;
+    static constexpr bool VSM = PT == 48;   // V through shared memory
+};
+template <int HD, int PT> constexpr size_t ax_smem() {   // queries, scores / weights, K tile, V tile
+    return ((size_t) PT * HD + (size_t) PT * (AxShape<PT>::TILE + 4)) * 4 + (size_t) AxShape<PT>::TILE * (2 * HD + 16) * (AxShape<PT>::VSM ? 2 : 1);
+}
+// the blocks a launch needs over (row, slice of PT pairs): a row leads at most the rows from it on
+static int ax_slices(int T, int qpk, int PT) {
+    int n = 0;
+    for (int t = 0; t < T; ++t) n += ((T - t) * qpk + PT - 1) / PT;
+    return n;
+}
+// four int8 values as floats, exactly: the byte + 128 under the exponent of 2^23, less 2^23 + 128
+__device__ __forceinline__ void ax_int8x4(unsigned w, float* f) {
+    w ^= 0x80808080u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f[j] = fsub(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | j)), 8388736.0f);
+}
 
-template <int HD, int PT>
-__global__ void __launch_bounds__(AX_THREADS, PT <= 16 ? 2 : 1) k_attn_rows(const float* __restrict__ qg, const uint16_t* __restrict__ kc,
+template <int HD, int PT, bool Q8>
+__global__ void __launch_bounds__(AxShape<PT>::THREADS, AxShape<PT>::BLOCKS) k_attn_rows(const float* __restrict__ qg, const uint16_t* __restrict__ kc,
                                                            const uint16_t* __restrict__ vc, FnxKvPages g, float* __restrict__ acc_out,
                                                            AttPart* __restrict__ mz_out, int T, int nq, int nkv,
                                                            const int* __restrict__ pos0p, int card, int ncard, FnxLaneRows lr,
                                                            const int* __restrict__ cells, const int* __restrict__ n_cells, int maxsel, int which) {
-    constexpr int G = AX_THREADS / HD, APT = PT / G, PPW = PT / AX_WARPS, KLD = HD + 4;   // thread groups over the pairs; accumulators a thread
-    const int s = blockIdx.x, kvl = blockIdx.y, lead = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int THREADS = AxShape<PT>::THREADS, WARPS = THREADS / 32, TILE = AxShape<PT>::TILE, QW = AxShape<PT>::QW, VD = AxShape<PT>::VD;
+    constexpr int SLD = TILE + 4;                                 // a pair's row of scores (16-byte aligned for the values' reads)
+    constexpr int KB = Q8 ? HD + HD / 16 + (HD == 128 ? 8 : 0) : 2 * HD + 16;   // bytes of a staged K row (int8: values, then scales): 16 past a multiple of 128
+    constexpr int VP = PT * (HD / VD) / THREADS;                  // pairs of a thread's accumulators
+    constexpr int PPW = PT / WARPS;                               // pairs of a warp's softmax steps
+    constexpr int QG = QW % 6 ? QW : 6, VG = VP % 6 ? VP : 6;     // pairs whose queries / weights are in registers together
+    constexpr bool VSM = AxShape<PT>::VSM;
+    static_assert(PT % WARPS == 0 && TILE / 64 * (PT / QW) == WARPS && TILE % 64 == 0 && KB % 128 == 16, "shape");
+    const int s = blockIdx.x, kvl = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int qpk = nq / nkv;
+    int lead = 0, slice = blockIdx.z;
+    for (int n; slice >= (n = ((T - lead) * qpk + PT - 1) / PT); ++lead) slice -= n;
     if (which && (cells && n_cells[lead] >= 0) != (which == 2)) return;   // this launch takes the other kind of rows
-    __shared__ int ctx_s[FNX_MAXT], len_s[FNX_MAXT], rows_s[FNX_MAXT], list_s[FNX_MAXT], nr_s;
+    __shared__ int ctx_s[FNX_MAXT], len_s[FNX_MAXT], rows_s[FNX_MAXT], list_s[FNX_MAXT], end_s[PT], nr_s;   // end_s: where a pair's run ends
     __shared__ const int* pt_s[FNX_MAXT];
     if (tid < T) {
         const bool listed = cells && n_cells[tid] >= 0;   // the row attends a list of its own (the block selection's)
@@ -160,165 +194,292 @@ __global__ void __launch_bounds__(AX_THREADS, PT <= 16 ? 2 : 1) k_attn_rows(cons
         nr_s = first && !(which == 1 && list_s[lead]) && !(which == 2 && !list_s[lead]) ? nr : 0;
     }
     __syncthreads();
-    const int nr = nr_s;
-    if (nr == 0) return;   // an earlier row leads this row's group
+    const int npairs = nr_s * qpk, nsl = (npairs + PT - 1) / PT;
+    if (slice >= nsl) return;   // an earlier row leads this row's group, or the group has fewer pairs
+    const int per = (npairs + 12 * nsl - 1) / (12 * nsl) * 12, pb = slice * per, npt = min(per, npairs - pb);   // slices of equal work
+    if (npt <= 0) return;
     g.pt = pt_s[lead];
     const int len = len_s[lead], p0 = s * len;
     const int* list = list_s[lead] ? cells + (size_t) lead * maxsel : nullptr;
-    int pend = 0;          // where the group's longest row ends inside this run
-    for (int r = 0; r < nr; ++r) pend = max(pend, min(ctx_s[rows_s[r]], p0 + len));
+    int pend = 0, pfull = 0x7fffffff;   // where the slice's longest row ends inside this run, and its shortest
+    for (int r = pb / qpk; r <= (pb + npt - 1) / qpk; ++r) {
+        const int e = min(ctx_s[rows_s[r]], p0 + len);
+        pend = max(pend, e), pfull = min(pfull, e);
+    }
+    if (tid < PT) end_s[tid] = tid < npt ? min(ctx_s[rows_s[(pb + tid) / qpk]], p0 + len) : 0;   // slots past the last pair: nothing
     extern __shared__ __align__(16) float ax_sm[];
-    float* q_s = ax_sm;                          // [PT][HD]
-    float* k_s = q_s + (size_t) PT * HD;      // [32][HD + 4]
-    float* v_s = k_s + (size_t) ATT_CH * KLD;    // [32][HD]
-    float* w_s = v_s + (size_t) ATT_CH * HD;     // [PT][32]
-    float* sc_s = w_s + (size_t) PT * ATT_CH; // [PT]
-    int* np_s = reinterpret_cast<int*>(sc_s + PT);   // [PT]: positions of the chunk the pair takes (0: none)
-    const float rs = ex_rsqrt((float) HD);
-    const int grp = tid / HD, d = tid % HD;
-    const int npairs = nr * qpk;
-#pragma unroll 1
-    for (int pb = 0; pb < npairs; pb += PT) {
-        const int npt = min(PT, npairs - pb);
-        __syncthreads();
-        for (int e = tid; e < npt * (HD / 4); e += AX_THREADS) {
-            const int pi = e / (HD / 4), c4 = e % (HD / 4), t = rows_s[(pb + pi) / qpk], h = kvl * qpk + (pb + pi) % qpk;
-            reinterpret_cast<float4*>(q_s + (size_t) pi * HD)[c4] = reinterpret_cast<const float4*>(qg + ((size_t) t * nq + h) * 2 * HD)[c4];
+    float* q_s = ax_sm;                            // [PT][HD]
+    float* s_s = q_s + (size_t) PT * HD;           // [PT][SLD] scores, then weights
+    unsigned char* k_s = reinterpret_cast<unsigned char*>(s_s + (size_t) PT * SLD);   // [TILE][KB] K rows as stored
+    unsigned char* v_s = k_s + (size_t) TILE * KB;   // [TILE][KB] V rows as stored (VSM)
+    __shared__ float sc_s[TILE / ATT_CH][PT];      // rescale factors
+    __shared__ int np_s[TILE / ATT_CH][PT];        // positions of a chunk the pair takes
+    __shared__ size_t at_s[2][TILE], sca_s[Q8 ? 2 : 1][Q8 ? TILE : 1];   // a tile's rows in the cache (halves, or bytes of int8 rows) and their scales
+    for (int e = tid; e < PT * (HD / 4); e += THREADS) {   // slots past the last pair repeat it; they are not written out
+        const int pi = e / (HD / 4), c4 = e % (HD / 4), p = pb + min(pi, npt - 1), t = rows_s[p / qpk], h = kvl * qpk + p % qpk;
+        reinterpret_cast<float4*>(q_s + (size_t) pi * HD)[c4] = reinterpret_cast<const float4*>(qg + ((size_t) t * nq + h) * 2 * HD)[c4];
+    }
+    auto locate = [&](int c0, int b) {
+        if (tid < TILE && p0 < pend) {   // positions past the end: the last one again (read, never used)
+            const int at = min(c0 + tid, pend - 1), r = list ? list[at] : at;
+            at_s[b][tid] = (Q8 ? kvq_row_at(g, r, nkv, HD) : kv_row_at(g, r, nkv, HD)) + (size_t) kvl * HD;
+            if (Q8) sca_s[b][tid] = kvq_scale_at(g, r, nkv, HD) + (size_t) kvl * (HD / 32);
         }
-        float m[PPW], z[PPW];
+    };
+    auto copy_rows = [&](const uint16_t* __restrict__ cache, unsigned char* dst_s, int c0, int b) {   // asynchronous; rows past the end are left as they are
+        constexpr int N = Q8 ? HD / 8 + HD / 128 : HD / 8;   // pieces a row: int8 8 bytes each, the scales' after the values'; f16 16 bytes
+        for (int e = tid; e < TILE * N; e += THREADS) {
+            const int pp = e / N, i = e % N;
+            if (c0 + pp >= pend) break;
+            const unsigned dst = um_s32(dst_s + (size_t) pp * KB) + (Q8 ? 8 : 16) * i;
+            if (Q8) {
+                const unsigned char* src = i < HD / 8 ? reinterpret_cast<const unsigned char*>(cache) + at_s[b][pp] + 8 * i
+                                                      : reinterpret_cast<const unsigned char*>(cache + sca_s[b][pp]) + 8 * (i - HD / 8);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src));
+            } else {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(cache + at_s[b][pp] + 8 * i));
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const float rs = ex_rsqrt((float) HD);
+    float m[PPW], z[PPW];   // the warp's pairs PPW warp .. + PPW - 1 (every lane the same)
 #pragma unroll
-        for (int i = 0; i < PPW; ++i) m[i] = -INFINITY, z[i] = 0.f;
-        float acc[APT];
+    for (int i = 0; i < PPW; ++i) m[i] = -INFINITY, z[i] = 0.f;
+    float acc[VP][VD];
 #pragma unroll
-        for (int i = 0; i < APT; ++i) acc[i] = 0.f;
+    for (int i = 0; i < VP; ++i)
+#pragma unroll
+        for (int k = 0; k < VD; ++k) acc[i][k] = 0.f;
+    const int vd = tid % (HD / VD) * VD, vg = tid / (HD / VD) * VP;      // values: first dimension, first pair
+    const int sp = warp / (PT / QW) * 64 + lane, sq = warp % (PT / QW) * QW;   // scores: positions sp and sp + 32, first pair
+    locate(p0, 0);
+    __syncthreads();
+    copy_rows(kc, k_s, p0, 0);
+    int b = 0;
 #pragma unroll 1
-        for (int c0 = p0; c0 < pend; c0 += ATT_CH) {
-            const int npmax = min(ATT_CH, pend - c0);
-            __syncthreads();   // the chunk before has been used up
-            // ---- the chunk's K and V rows as f32: 16-byte pieces of 8 halves
-            for (int e = tid; e < ATT_CH * (HD / 8); e += AX_THREADS) {
-                const int pp = e / (HD / 8), c8 = e % (HD / 8);
-                float kf[8], vf[8];
-                if (g.q8) {   // int8 values times their group's scale (reference src/kernels.cu:531-537): 8 values of one group
-                    uint2 kr = make_uint2(0, 0), vr = kr;
-                    float kd8 = 0.f, vd8 = 0.f;
-                    if (pp < npmax) {
-                        const int r = list ? list[c0 + pp] : c0 + pp;
-                        const size_t at = kvq_row_at(g, r, nkv, HD) + (size_t) kvl * HD + 8 * c8;
-                        const size_t sc = kvq_scale_at(g, r, nkv, HD) + ((size_t) kvl * HD + 8 * c8) / 32;
-                        kr = *reinterpret_cast<const uint2*>(reinterpret_cast<const int8_t*>(kc) + at);
-                        vr = *reinterpret_cast<const uint2*>(reinterpret_cast<const int8_t*>(vc) + at);
-                        kd8 = h2f(kc[sc]), vd8 = h2f(vc[sc]);
-                    }
-                    const unsigned kw[2] = {kr.x, kr.y}, vw[2] = {vr.x, vr.y};
+    for (int c0 = p0; c0 < pend; c0 += TILE, b ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // the tile's K rows are in place; the tile before is used up
+        if (VSM) copy_rows(vc, v_s, c0, b);
+        locate(c0 + TILE, b ^ 1);
+        if (sq < npt) {   // ---- scores
+            float sa[2][QW];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        kf[k] = fmul((float) (int8_t) (kw[k >> 2] >> (8 * (k & 3))), kd8);
-                        vf[k] = fmul((float) (int8_t) (vw[k >> 2] >> (8 * (k & 3))), vd8);
-                    }
-                } else {
-                    uint4 kr = make_uint4(0, 0, 0, 0), vr = kr;
-                    if (pp < npmax) {
-                        const size_t at = kv_row_at(g, list ? list[c0 + pp] : c0 + pp, nkv, HD) + (size_t) kvl * HD + 8 * c8;
-                        kr = *reinterpret_cast<const uint4*>(kc + at);
-                        vr = *reinterpret_cast<const uint4*>(vc + at);
-                    }
-                    const unsigned kw[4] = {kr.x, kr.y, kr.z, kr.w}, vw[4] = {vr.x, vr.y, vr.z, vr.w};
+            for (int i = 0; i < QW; ++i) sa[0][i] = sa[1][i] = 0.f;
+            const unsigned char* kp = k_s + (size_t) sp * KB;
+            const float* qp = q_s + (size_t) sq * HD;
+            float qq[2][QG][4];
+            auto read_q = [&](int u, int gi, int c) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        kf[2 * k] = h2f((uint16_t) (kw[k] & 0xffff)), kf[2 * k + 1] = h2f((uint16_t) (kw[k] >> 16));
-                        vf[2 * k] = h2f((uint16_t) (vw[k] & 0xffff)), vf[2 * k + 1] = h2f((uint16_t) (vw[k] >> 16));
+                for (int i = 0; i < QG; ++i) *reinterpret_cast<float4*>(qq[u][i]) = *reinterpret_cast<const float4*>(qp + (size_t) (gi * QG + i) * HD + c);
+            };
+            read_q(0, 0, 0);
+            // 16 dimensions a step: two reads of 8 f16 values, or one of 16 int8 values
+            uint4 kr[2][2], kn[2][2];
+            auto read_k = [&](uint4 (&r)[2][2], int c) {
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const uint4* a = reinterpret_cast<const uint4*>(kp + (size_t) 32 * p * KB + (Q8 ? 1 : 2) * c);
+                    r[p][0] = a[0];
+                    if (!Q8) r[p][1] = a[1];
+                }
+            };
+            read_k(kr, 0);
+            float kd[2] = {0.f, 0.f};
+#pragma unroll 1
+            for (int c = 0; c < HD; c += 16) {
+                if (c + 16 < HD) read_k(kn, c + 16);
+                if (Q8 && (c & 31) == 0) {
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) kd[p] = h2f(*reinterpret_cast<const uint16_t*>(kp + (size_t) 32 * p * KB + HD + c / 16));
+                }
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {   // 4 dimensions
+                    float kf[2][4];
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        if (Q8) {   // int8 values times their group's scale (reference src/kernels.cu:531-537)
+                            ax_int8x4(h == 0 ? kr[p][0].x : h == 1 ? kr[p][0].y : h == 2 ? kr[p][0].z : kr[p][0].w, kf[p]);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) kf[p][e] = fmul(kf[p][e], kd[p]);
+                        } else {
+                            const uint4 w = kr[p][h >> 1];
+                            const unsigned lo = h & 1 ? w.z : w.x, hi = h & 1 ? w.w : w.y;
+                            kf[p][0] = h2f((uint16_t) (lo & 0xffff)), kf[p][1] = h2f((uint16_t) (lo >> 16));
+                            kf[p][2] = h2f((uint16_t) (hi & 0xffff)), kf[p][3] = h2f((uint16_t) (hi >> 16));
+                        }
+                    }
+#pragma unroll
+                    for (int gi = 0; gi < QW / QG; ++gi) {
+                        constexpr int NG = QW / QG;
+                        const int u = (h * NG + gi) & 1;
+                        if (gi + 1 < NG) read_q(u ^ 1, gi + 1, c + 4 * h);
+                        else read_q(u ^ 1, 0, min(c + 4 * h + 4, HD - 4));   // (the very last: read again, not used)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+#pragma unroll
+                            for (int i = 0; i < QG; ++i)
+#pragma unroll
+                                for (int p = 0; p < 2; ++p) sa[p][gi * QG + i] = ffma(qq[u][i][e], kf[p][e], sa[p][gi * QG + i]);
                     }
                 }
-                float4* kd = reinterpret_cast<float4*>(k_s + (size_t) pp * KLD + 8 * c8);
-                float4* vd = reinterpret_cast<float4*>(v_s + (size_t) pp * HD + 8 * c8);
-                kd[0] = make_float4(kf[0], kf[1], kf[2], kf[3]), kd[1] = make_float4(kf[4], kf[5], kf[6], kf[7]);
-                vd[0] = make_float4(vf[0], vf[1], vf[2], vf[3]), vd[1] = make_float4(vf[4], vf[5], vf[6], vf[7]);
-            }
-            __syncthreads();
-            // ---- scores: this lane's position against the warp's pairs, each a fused chain over the head dimension
-            float sa[PPW];
 #pragma unroll
-            for (int i = 0; i < PPW; ++i) sa[i] = 0.f;
-            const float4* k4 = reinterpret_cast<const float4*>(k_s + (size_t) lane * KLD);
-#pragma unroll 2
-            for (int c4 = 0; c4 < HD / 4; ++c4) {
-                const float4 kk = k4[c4];
+                for (int p = 0; p < 2; ++p) kr[p][0] = kn[p][0], kr[p][1] = kn[p][1];
+            }
+#pragma unroll
+            for (int i = 0; i < QW; ++i) s_s[(size_t) (sq + i) * SLD + sp] = sa[0][i], s_s[(size_t) (sq + i) * SLD + sp + 32] = sa[1][i];
+        }
+        __syncthreads();   // scores are written, K is used up
+        if (c0 + TILE < pend) copy_rows(kc, k_s, c0 + TILE, b ^ 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        // ---- V: a thread's VD values of a position as stored (int8: with their scale above them)
+        auto read_v = [&](uint2& r, int pp) {
+            if (VSM) {
+                const unsigned char* a = v_s + (size_t) pp * KB + (Q8 ? 1 : 2) * vd;
+                if (Q8) r.x = *reinterpret_cast<const unsigned*>(a), r.y = *reinterpret_cast<const uint16_t*>(v_s + (size_t) pp * KB + HD + vd / 32 * 2);
+                else r = *reinterpret_cast<const uint2*>(a);
+            } else if (Q8) {
+                const unsigned v = __ldg(reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(vc) + at_s[b][pp] + vd));
+                r.x = v | (unsigned) __ldg(vc + sca_s[b][pp] + vd / 32) << 16;
+            } else {
+                r.x = __ldg(reinterpret_cast<const unsigned*>(vc + at_s[b][pp] + vd));
+            }
+        };
+        auto unpack_v = [&](const uint2& r, float* f) {
+            if (Q8) {
+                float t[4];
+                const float d = h2f((uint16_t) (VSM ? r.y : r.x >> 16));
+                ax_int8x4(r.x, t);
+#pragma unroll
+                for (int k = 0; k < VD; ++k) f[k] = fmul(t[k], d);
+            } else {
+                f[0] = h2f((uint16_t) (r.x & 0xffff)), f[1] = h2f((uint16_t) (r.x >> 16));
+                if (VD == 4) f[VD - 2] = h2f((uint16_t) (r.y & 0xffff)), f[VD - 1] = h2f((uint16_t) (r.y >> 16));
+            }
+        };
+        const bool has_v = vg < npt;
+        uint2 vr[VSM ? 1 : TILE];   // narrow: the whole tile's, on their way while the softmax steps are taken
+        if (!VSM && has_v) {
+#pragma unroll
+            for (int k = 0; k < TILE; ++k) read_v(vr[VSM ? 0 : k], k);
+        }
+        // ---- the online-softmax steps of the warp's pairs, two chunks at a time (a pair without positions in a chunk gets a
+        // factor of exactly one, or of zero on an empty sum, and weights of zero)
+#pragma unroll 1
+        for (int cc = 0; cc < TILE / ATT_CH; cc += 2) {
+            float mx[2][PPW], sv[2][PPW], sc[2][PPW];
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int i = 0; i < PPW; ++i) {
-                    const float4 qq = reinterpret_cast<const float4*>(q_s + (size_t) (warp + AX_WARPS * i) * HD)[c4];
-                    sa[i] = ffma(qq.x, kk.x, sa[i]);
-                    sa[i] = ffma(qq.y, kk.y, sa[i]);
-                    sa[i] = ffma(qq.z, kk.z, sa[i]);
-                    sa[i] = ffma(qq.w, kk.w, sa[i]);
+                    const int pi = PPW * warp + i, np = min(ATT_CH, end_s[pi] - c0 - (cc + c) * ATT_CH);
+                    sv[c][i] = lane < np ? fmul(s_s[(size_t) pi * SLD + (cc + c) * ATT_CH + lane], rs) : -INFINITY;
+                    if (lane == 0) np_s[cc + c][pi] = np;
                 }
-            }
-            // ---- the online-softmax step of every pair of the warp (all lanes hold the pair's m and z)
 #pragma unroll
-            for (int i = 0; i < PPW; ++i) {
-                const int pi = warp + AX_WARPS * i;
-                if (pi < npt) {
-                    const int t = rows_s[(pb + pi) / qpk];
-                    const int np = min(ATT_CH, min(ctx_s[t], p0 + len) - c0);   // <= 0: this row's run ended before the chunk
-                    if (np > 0) {
-                        const float sv = lane < np ? fmul(sa[i], rs) : -INFINITY;
-                        const float mn = fmaxf(m[i], wmax(sv));
-                        const float w = sv == -INFINITY ? 0.f : ex_expf(fsub(sv, mn));
-                        const float sc = m[i] == -INFINITY ? 0.f : ex_expf(fsub(m[i], mn));
-                        z[i] = ffma(z[i], sc, wsum(w));
-                        m[i] = mn;
-                        w_s[pi * ATT_CH + lane] = w;
-                        if (lane == 0) sc_s[pi] = sc;
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int i = 0; i < PPW; ++i) asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx[c][i]) : "f"(sv[c][i]));   // a maximum is the same in any order
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int i = 0; i < PPW; ++i) {
+                    const int pi = PPW * warp + i;
+                    const float mn = fmaxf(m[i], mx[c][i]);
+                    sv[c][i] = sv[c][i] == -INFINITY ? 0.f : ex_expf(fsub(sv[c][i], mn));
+                    sc[c][i] = m[i] == -INFINITY ? 0.f : ex_expf(fsub(m[i], mn));
+                    m[i] = mn;
+                    s_s[(size_t) pi * SLD + (cc + c) * ATT_CH + lane] = sv[c][i];
+                    if (lane == 0) sc_s[cc + c][pi] = sc[c][i];
+                }
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int i = 0; i < PPW; ++i) sv[c][i] = fadd(sv[c][i], __shfl_xor_sync(0xffffffffu, sv[c][i], o));
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int i = 0; i < PPW; ++i) z[i] = ffma(z[i], sc[c][i], sv[c][i]);
+        }
+        if (VSM) asm volatile("cp.async.wait_group 1;" ::: "memory");   // V has landed (the next tile's K may be on its way)
+        __syncthreads();   // weights and factors are in place
+        // ---- values: acc = acc sc, then + w v in ascending position
+        if (has_v) {
+            const int live = min(TILE, pend - c0);
+            auto four = [&](int pp0, int j) {   // positions pp0 .. + 3 of the tile; j: pp0 where it is a constant (the registers of a narrow block)
+                const int c = pp0 / ATT_CH;
+                if (pp0 % ATT_CH == 0) {
+#pragma unroll
+                    for (int i = 0; i < VP; ++i) {
+                        const float sc = sc_s[c][vg + i];
+#pragma unroll
+                        for (int k = 0; k < VD; ++k) acc[i][k] = fmul(acc[i][k], sc);
                     }
-                    if (lane == 0) np_s[pi] = max(np, 0);
                 }
-            }
-            __syncthreads();
-            // ---- values: acc = acc sc, then + w v in ascending position, for this thread's dimension
-            float vv[ATT_CH];
+                float v[4][VD];
 #pragma unroll
-            for (int pp = 0; pp < ATT_CH; ++pp) vv[pp] = v_s[(size_t) pp * HD + d];
+                for (int k = 0; k < 4; ++k) {
+                    uint2 r;
+                    if (VSM) read_v(r, pp0 + k);
+                    else r = vr[VSM ? 0 : j + k];
+                    unpack_v(r, v[k]);
+                }
+                const bool whole = c0 + (c + 1) * ATT_CH <= pfull;   // every pair takes the whole chunk
 #pragma unroll
-            for (int i = 0; i < APT; ++i) {
-                const int pi = grp * APT + i;
-                if (pi < npt) {
-                    const int np = np_s[pi];
-                    if (np == ATT_CH) {
-                        float a = fmul(acc[i], sc_s[pi]);
-                        const float4* w4 = reinterpret_cast<const float4*>(w_s + (size_t) pi * ATT_CH);
+                for (int gi = 0; gi < VP / VG; ++gi) {
+                    float w[VG][4];
 #pragma unroll
-                        for (int p4 = 0; p4 < ATT_CH / 4; ++p4) {
-                            const float4 ww = w4[p4];
-                            a = ffma(ww.x, vv[4 * p4], a);
-                            a = ffma(ww.y, vv[4 * p4 + 1], a);
-                            a = ffma(ww.z, vv[4 * p4 + 2], a);
-                            a = ffma(ww.w, vv[4 * p4 + 3], a);
+                    for (int i = 0; i < VG; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(s_s + (size_t) (vg + gi * VG + i) * SLD + pp0);
+                    if (whole) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+#pragma unroll
+                            for (int i = 0; i < VG; ++i)
+#pragma unroll
+                                for (int d = 0; d < VD; ++d) acc[gi * VG + i][d] = ffma(w[i][k], v[k][d], acc[gi * VG + i][d]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < VG; ++i) {
+                            const int np = np_s[c][vg + gi * VG + i] - pp0 % ATT_CH;
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                if (k < np) {
+#pragma unroll
+                                    for (int d = 0; d < VD; ++d) acc[gi * VG + i][d] = ffma(w[i][k], v[k][d], acc[gi * VG + i][d]);
+                                }
                         }
-                        acc[i] = a;
-                    } else if (np > 0) {   // a row's last, partial chunk
-                        float a = fmul(acc[i], sc_s[pi]);
-                        for (int pp = 0; pp < np; ++pp) a = ffma(w_s[pi * ATT_CH + pp], v_s[(size_t) pp * HD + d], a);
-                        acc[i] = a;
                     }
                 }
+            };
+            if (VSM) {
+#pragma unroll 2
+                for (int p = 0; p < live; p += 4) four(p, 0);
+            } else {
+#pragma unroll
+                for (int p = 0; p < TILE; p += 4)
+                    if (p < live) four(p, p);
             }
         }
-        // ---- this run's partial of every pair of the tile
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // ---- this run's partial of every pair
 #pragma unroll
-        for (int i = 0; i < APT; ++i) {
-            const int pi = grp * APT + i;
-            if (pi < npt) {
-                const int t = rows_s[(pb + pi) / qpk], h = kvl * qpk + (pb + pi) % qpk;
-                acc_out[(((size_t) t * nq + h) * ATT_SPLITS + s) * HD + d] = acc[i];
-            }
+    for (int i = 0; i < VP; ++i)
+        if (vg + i < npt) {
+            const int p = pb + vg + i, t = rows_s[p / qpk], h = kvl * qpk + p % qpk;
+#pragma unroll
+            for (int k = 0; k < VD; k += 2)
+                *reinterpret_cast<float2*>(acc_out + (((size_t) t * nq + h) * ATT_SPLITS + s) * HD + vd + k) = make_float2(acc[i][k], acc[i][k + 1]);
         }
 #pragma unroll
-        for (int i = 0; i < PPW; ++i) {
-            const int pi = warp + AX_WARPS * i;
-            if (pi < npt && lane == 0) {
-                const int t = rows_s[(pb + pi) / qpk], h = kvl * qpk + (pb + pi) % qpk;
-                mz_out[((size_t) t * nq + h) * ATT_SPLITS + s] = AttPart{m[i], z[i]};
-            }
+    for (int i = 0; i < PPW; ++i) {
+        const int pi = PPW * warp + i;
+        if (pi < npt && lane == 0) {
+            const int t = rows_s[(pb + pi) / qpk], h = kvl * qpk + (pb + pi) % qpk;
+            mz_out[((size_t) t * nq + h) * ATT_SPLITS + s] = AttPart{m[i], z[i]};
         }
     }
 }
@@ -591,15 +752,19 @@ static int attn_partial_rows(const float* qg, const uint16_t* kc, const uint16_t
     FNX_REQUIRE(!g.q8 || lr.pt || g.pt || g.cap > 0, "attn: an int8 cache without a page table needs its row count (cap)");
     float* acc = scratch;
     AttPart* mz = (AttPart*) (scratch + (size_t) T * nq * ATT_SPLITS * hd);
-    const dim3 grid(ATT_SPLITS, nkv, T);   // block z = t works only when row t leads a group of rows
-    auto run = [&](auto kern, int pt, int which) -> int {
-        const size_t sm = ((size_t) pt * hd + (size_t) ATT_CH * (hd + 4) + (size_t) ATT_CH * hd + (size_t) pt * ATT_CH + 2 * pt) * sizeof(float);
+    const int qpk = nq / nkv;
+    const dim3 grid(ATT_SPLITS, nkv, T);
+    auto run = [&](auto kern, int PT, int threads, size_t sm, int which) -> int {   // the rows' groups, in slices of PT pairs
         if (smem_optin(kern, sm, "attn partial")) return 1;
-        kern<<<grid, AX_THREADS, sm, strm(st)>>>(qg, kc, vc, g, acc, mz, T, nq, nkv, pos0, card, ncard, lr, cells, n_cells, maxsel, which);
+        kern<<<dim3(ATT_SPLITS, nkv, ax_slices(T, qpk, PT)), threads, sm, strm(st)>>>(qg, kc, vc, g, acc, mz, T, nq, nkv, pos0, card, ncard, lr, cells,
+                                                                                     n_cells, maxsel, which);
         return 0;
     };
+#define AX_RUN(HD, PT, which)                                                                          \
+    (g.q8 ? run(k_attn_rows<HD, PT, true>, PT, AxShape<PT>::THREADS, ax_smem<HD, PT>(), which)         \
+          : run(k_attn_rows<HD, PT, false>, PT, AxShape<PT>::THREADS, ax_smem<HD, PT>(), which))
     auto listed = [&](auto kern) -> int {   // rows with a list over an f16 cache: as many chunks a group as the longest run has, 8 at most
-        const int qpk = nq / nkv, len_max = ((maxsel + ATT_SPLITS - 1) / ATT_SPLITS + ATT_CH - 1) / ATT_CH * ATT_CH;
+        const int len_max = ((maxsel + ATT_SPLITS - 1) / ATT_SPLITS + ATT_CH - 1) / ATT_CH * ATT_CH;
         const int nch = len_max / ATT_CH < AX_WARPS ? len_max / ATT_CH : AX_WARPS;
         const size_t sm = (size_t) qpk * hd * 4 + (size_t) nch * ATT_CH * (hd + 8) * 2 + (size_t) nch * qpk * ATT_CH * 4 + (size_t) 3 * nch * qpk * 4 +
                           (size_t) (2 * qpk + 2) * 4 + (size_t) nch * ATT_CH * sizeof(size_t) + 16;
@@ -609,17 +774,19 @@ static int attn_partial_rows(const float* qg, const uint16_t* kc, const uint16_t
         kern<<<grid, AX_THREADS, sm, strm(st)>>>(qg, kc, vc, g, acc, mz, nq, nkv, lr, cells, n_cells, maxsel, nch, fault);
         return 0;
     };
-    // rows with a list of their own go in a launch of their own; the others in groups of up to 96 pairs
-    const bool small = nq / nkv <= 8;
+    // rows with a list of their own go in a launch of their own.  Wide slices when the rows are one sequence's and make
+    // more than a narrow one; narrow ones for rows of several sequences, whose groups are small
+    const bool few = qpk <= 8, wide = !lr.pos && T * qpk > 12;
     if (hd == 256) {
-        if (run(k_attn_rows<256, AX_PT>, AX_PT, cells ? 1 : 0)) return 1;
-        if (cells && g.q8 && (small ? run(k_attn_rows<256, 8>, 8, 2) : run(k_attn_rows<256, 16>, 16, 2))) return 1;
-        if (cells && !g.q8 && (small ? listed(k_attn_cells<256, 8>) : listed(k_attn_cells<256, 16>))) return 1;
+        if (wide ? AX_RUN(256, 48, cells ? 1 : 0) : AX_RUN(256, 12, cells ? 1 : 0)) return 1;
+        if (cells && g.q8 && AX_RUN(256, 12, 2)) return 1;
+        if (cells && !g.q8 && (few ? listed(k_attn_cells<256, 8>) : listed(k_attn_cells<256, 16>))) return 1;
     } else {
-        if (run(k_attn_rows<128, AX_PT>, AX_PT, cells ? 1 : 0)) return 1;
-        if (cells && g.q8 && (small ? run(k_attn_rows<128, 8>, 8, 2) : run(k_attn_rows<128, 16>, 16, 2))) return 1;
-        if (cells && !g.q8 && (small ? listed(k_attn_cells<128, 8>) : listed(k_attn_cells<128, 16>))) return 1;
+        if (wide ? AX_RUN(128, 48, cells ? 1 : 0) : AX_RUN(128, 12, cells ? 1 : 0)) return 1;
+        if (cells && g.q8 && AX_RUN(128, 12, 2)) return 1;
+        if (cells && !g.q8 && (few ? listed(k_attn_cells<128, 8>) : listed(k_attn_cells<128, 16>))) return 1;
     }
+#undef AX_RUN
     if (launch_ok("attn partial")) return 1;
     k_attn_join_runs<<<dim3(T, nq), 256, 0, strm(st)>>>(acc, mz, part, nq, hd);
     return launch_ok("attn join");

@@ -21,10 +21,11 @@ int q8s_umma_launch(const FnxQ8S* w, const int* rows, float* const* out, const i
 unsigned* device_fault_word();
 void fault_sink(unsigned* err);
 
-// shared memory past the default 48 KB has to be asked for, once per kernel
+// shared memory past the default 48 KB has to be asked for, once per kernel (a kernel's static arrays, at most 16 KB here,
+// count against the 48 KB too)
 template <typename K> int smem_optin(K kernel, size_t bytes, const char* what) {
     if (bytes > 227 * 1024) return fail("%s: %zu bytes of shared memory exceed an SM's 227 KB", what, bytes);
-    if (bytes > 48 * 1024) {
+    if (bytes > 32 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
         if (e != cudaSuccess) return fail("%s: shared memory opt-in: %s", what, cudaGetErrorString(e));
     }

@@ -79,6 +79,19 @@ def test_attention_int8_kv(T, ctx, ncard, hd):
         assert np.array_equal(got["out"].view(np.uint32), ref["out"].view(np.uint32)), "merged, gated output"
 
 
+@pytest.mark.parametrize("q8", [False, True])
+@pytest.mark.parametrize("T,ctx,hd", [(16, 505, 256), (9, 1020, 256), (2, 511, 256), (11, 4100, 256), (16, 1021, 128), (3, 31, 128)])
+def test_attention_exact_rows_in_groups_and_slices(T, ctx, hd, q8):
+    """The exact-order scan where rows of one window fall into two groups (the runs' length changes inside the window), groups
+    make one, two or unequal slices of pairs (12 to 96 pairs), and runs end inside a staged tile or a chunk; f16 and int8
+    rows, bit for bit."""
+    c = cases.attn_case(T=T, ctx=ctx, nq=12 if hd == 128 else 24, nkv=2 if hd == 128 else 4, hd=hd, seed=40 + T)
+    if q8:
+        c = cases.attn_case_q8(c)
+    ref, got = cases.attn_oracle(c), _run(c, "fnx_attn_partial_exact")
+    assert np.array_equal(got["part"][0].view(np.uint32), ref["part"][0].view(np.uint32))
+
+
 @pytest.mark.parametrize("T,ctx,ncard,hd", [(16, 3000, 1, 256), (16, 70, 1, 256), (7, 1500, 2, 256), (5, 515, 4, 128), (1, 0, 1, 256),
                                             (16, 40000, 1, 256), (2, 262144, 1, 256), (3, 70000, 8, 256)])
 @pytest.mark.parametrize("known_rows", [False, True])
