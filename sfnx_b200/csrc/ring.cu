@@ -153,7 +153,7 @@ struct BoundaryArgs {
     float eps;
     unsigned* err;
 };
-constexpr int BD_THREADS = 1024, BD_MAXN = 4096, BD_CL = 8, BD_CT = BD_THREADS / BD_CL, BD_MAXC = BD_MAXN / BD_THREADS;
+constexpr int BD_THREADS = 1024, BD_MAXN = 4096, BD_CL = 8, BD_CT = BD_THREADS / BD_CL, BD_MAXC = BD_MAXN / BD_THREADS, BD_KK = 10;
 
 __device__ __forceinline__ void bd_q8_1_store(float xi, uint8_t* blk, int lane) {
     const float amax = wmax(fabsf(xi)), sum = wsum(xi);
@@ -175,25 +175,49 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_CT) k_boundar
     const int t = blockIdx.x / BD_CL, cr = blockIdx.x % BD_CL, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int vt = cr * BD_CT + tid, n = a.n, nr = a.ring.nrank, me = a.ring.rank;
     float* xr = a.x + (size_t) t * n;
+    float wv[BD_MAXC];   // the norm's weights do not depend on the kernel ahead
+#pragma unroll
+    for (int k = 0; k < BD_MAXC; ++k) wv[k] = __ldg(a.w + min(vt + BD_THREADS * k, n - 1));
     pdl_wait();
     pdl_go();
     const bool has_add = a.bo || a.moe.part;
-    // ---- this GPU's addend of the row, this thread's columns
-    float add[BD_MAXC];
+    // ---- this GPU's addend of the row, this thread's columns.  The kernel is a chain of latencies, so everything a thread
+    // reads (x, and a column's ten expert rows) is asked for before the first of it is used.
+    float add[BD_MAXC], xo[BD_MAXC];
 #pragma unroll
-    for (int k = 0; k < BD_MAXC; ++k) add[k] = 0.f;
+    for (int k = 0; k < BD_MAXC; ++k) {
+        const int i = vt + BD_THREADS * k;
+        add[k] = 0.f;
+        xo[k] = i < n ? xr[i] : 0.f;
+    }
     if (a.moe.part) {
         const int topk = a.moe.topk;
-        const float gate = ex_sigmoid(a.moe.logits[(size_t) t * (a.moe.nexp + 1) + a.moe.nexp]);
+        const float lg = a.moe.logits[(size_t) t * (a.moe.nexp + 1) + a.moe.nexp];
+        float sh[BD_MAXC];
 #pragma unroll
-        for (int k = 0; k < BD_MAXC; ++k) {
-            const int i = vt + BD_THREADS * k;
-            if (i < n) {
-                float s = 0.f;
-                for (int kk = 0; kk < topk; ++kk) s = ffma(a.moe.topw[t * topk + kk], a.moe.part[((size_t) t * topk + kk) * n + i], s);
-                add[k] = ffma(gate, a.moe.sh[(size_t) t * n + i], s);
+        for (int k = 0; k < BD_MAXC; ++k) sh[k] = vt + BD_THREADS * k < n ? a.moe.sh[(size_t) t * n + vt + BD_THREADS * k] : 0.f;
+        for (int k0 = 0; k0 < topk; k0 += BD_KK) {   // ten rows of a column at a time, every column's before the first sum
+            const float tw = lane < BD_KK && k0 + lane < topk ? a.moe.topw[t * topk + k0 + lane] : 0.f;
+            float pv[BD_MAXC][BD_KK];
+#pragma unroll
+            for (int k = 0; k < BD_MAXC; ++k)
+#pragma unroll
+                for (int kk = 0; kk < BD_KK; ++kk) {
+                    const int i = vt + BD_THREADS * k;
+                    pv[k][kk] = i < n && k0 + kk < topk ? a.moe.part[((size_t) t * topk + k0 + kk) * n + i] : 0.f;
+                }
+#pragma unroll
+            for (int kk = 0; kk < BD_KK; ++kk) {
+                const float w = __shfl_sync(0xffffffffu, tw, kk);
+                if (k0 + kk < topk) {
+#pragma unroll
+                    for (int k = 0; k < BD_MAXC; ++k) add[k] = ffma(w, pv[k][kk], add[k]);
+                }
             }
         }
+        const float gate = ex_sigmoid(lg);
+#pragma unroll
+        for (int k = 0; k < BD_MAXC; ++k) add[k] = ffma(gate, sh[k], add[k]);
     } else if (a.bo) {
 #pragma unroll
         for (int k = 0; k < BD_MAXC; ++k) {
@@ -265,7 +289,7 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_CT) k_boundar
         const int i = vt + BD_THREADS * k;
         v[k] = 0.f;
         if (i < n) {
-            float val = xr[i];
+            float val = xo[k];
             if (has_add) {
                 val = fadd(val, add[k]);
                 xr[i] = val;
@@ -288,7 +312,7 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_CT) k_boundar
     for (int k = 0; k < BD_MAXC; ++k) {
         const int i = vt + BD_THREADS * k;
         if (i - lane < n) {   // warp-uniform: a warp's 32 columns are one q8_1 block (n is a multiple of 32)
-            const float val = fmul(fmul(v[k], r), a.w[i]);
+            const float val = fmul(fmul(v[k], r), wv[k]);
             if (a.y) a.y[(size_t) t * n + i] = val;
             if (a.q) bd_q8_1_store(val, a.q + ((size_t) t * (n / 32) + (i >> 5)) * 36, lane);
         }
