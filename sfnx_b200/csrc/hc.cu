@@ -19,7 +19,7 @@
 namespace fnxk {
 
 constexpr int HC_SL = 512, HC_RPG = 96, HC_TPR = 8, HC_DT = HC_RPG * HC_TPR, HC_MAXS = 8;   // slice; rows a group; lanes a row; streams
-constexpr int HC_UPC = 32, HC_TPU = 16, HC_UT = HC_UPC * HC_TPU;                           // up: columns a block, lanes a column
+constexpr int HC_UPC = 32, HC_TPU = 16, HC_UT = HC_UPC * HC_TPU, HC_UE = 4;                // up: columns a block, lanes a column
 
 struct HcArgs {
     float* R;
@@ -66,17 +66,27 @@ __global__ void k_hc_add_streams(const float* __restrict__ h, const float* __res
     if (j < n * hc) R[(size_t) t * n * hc + j] = fadd(h[(size_t) t * n * hc + j], e[(size_t) t * n + j % n]);
 }
 
-__device__ __forceinline__ float hc_rprime(const HcArgs& a, int t, int c, int i) {
-    float r = a.R[((size_t) t * a.hc + c) * a.n + i];
-    if (a.bo) r = ffma(a.bo[(size_t) t * a.n + i], fmul(2.0f, ex_sigmoid(fdiv(a.inj_prev[t * a.hc + c], (float) a.hc))), r);
-    return r;
+// R' = R + bo g, g the write's gate of row t, stream c
+__device__ __forceinline__ float hc_gate(const HcArgs& a, int t, int c) {
+    return fmul(2.0f, ex_sigmoid(fdiv(a.inj_prev[t * a.hc + c], (float) a.hc)));
 }
-__device__ __forceinline__ int hc_dot8(const uint2 w, const int2 x) { return __dp4a((int) w.y, x.y, __dp4a((int) w.x, x.x, 0)); }
+// integer dots are started at the bits of 1.5 * 2^23: as floats minus that, (float) dot, without a convert instruction
+// (a quarter of the rate of the multiply-adds; the dots stay under 2^22)
+constexpr int HC_MAGIC = 0x4B400000;
+__device__ __forceinline__ float hc_float(int dot) { return fsub(__int_as_float(dot), 12582912.0f); }
+__device__ __forceinline__ int hc_dot8(const uint2 w, const int2 x) { return __dp4a((int) w.y, x.y, __dp4a((int) w.x, x.x, HC_MAGIC)); }
 // rs of row k, stream c from the slices' square sums, the slices in ascending order
 __device__ __forceinline__ float hc_rs(const HcArgs& a, int k, int c) {
     const int ns = a.n * a.hc / HC_SL, sps = a.n / HC_SL;
     float v = 0.f;
-    for (int ss = 0; ss < sps; ++ss) v = fadd(v, a.ssp[(size_t) k * ns + c * sps + ss]);
+    for (int s0 = 0; s0 < sps; s0 += 8) {   // the loads of eight slices ahead of their ordered sum
+        float q[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q[i] = s0 + i < sps ? a.ssp[(size_t) k * ns + c * sps + s0 + i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (s0 + i < sps) v = fadd(v, q[i]);
+    }
     return ex_rsqrt(fadd(fdiv(v, (float) a.n), a.eps));
 }
 
@@ -116,17 +126,45 @@ __global__ void __launch_bounds__(HC_DT) k_hc_down(const HcArgs a) {
             wr[4 * q] = v.x, wr[4 * q + 1] = v.y, wr[4 * q + 2] = v.z, wr[4 * q + 3] = v.w;
         }
     }
+    const float wn = t < HC_SL ? __ldg(a.w_norm + col0 + t) : 0.f;
+    __shared__ float gate[FNX_MAXT];
     pdl_wait();
     pdl_go();
-    if (t < HC_SL) {
-        const float wn = a.w_norm[col0 + t];
-        for (int k = 0; k < T; ++k) {
-            const float r = hc_rprime(a, k, c, i0 + t);
-            xs[(size_t) k * HC_SL + t] = fmul(r, wn);
-            if (grp == 0) {   // block-uniform; warps 0..15 hold the slice
-                const float v = wsum(fmul(r, r));
-                if (lane == 0) red[k * (HC_SL / 32) + warp] = v;
-            }
+    if (a.bo && t >= HC_SL && t - HC_SL < T) gate[t - HC_SL] = hc_gate(a, t - HC_SL, c);
+    // Rows eight at a time: their loads go out together, then their warp sums and maxima interleave (a row at a time, each
+    // step of this chain is waited for T times).  Warp w < 16 holds the slice's 32-value block w of every row.
+    for (int k0 = 0; k0 < T; k0 += 8) {
+        float r[8], bv[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool in = t < HC_SL && k0 + i < T;
+            r[i] = in ? a.R[((size_t) (k0 + i) * a.hc + c) * a.n + i0 + t] : 0.f;
+            bv[i] = in && a.bo ? a.bo[(size_t) (k0 + i) * a.n + i0 + t] : 0.f;
+        }
+        if (k0 == 0) __syncthreads();   // the gates
+        if (t >= HC_SL) continue;
+        float sq[8], amax[8], v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (a.bo && k0 + i < T) r[i] = ffma(bv[i], gate[k0 + i], r[i]);
+            v[i] = fmul(r[i], wn);
+            amax[i] = fabsf(v[i]), sq[i] = fmul(r[i], r[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax[i] = wmax(amax[i]);
+        if (grp == 0) {   // block-uniform
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sq[i] = wsum(sq[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int k = k0 + i;
+            if (k >= T) break;
+            const float d = fdiv(amax[i], 127.0f);   // the block's float scale
+            xs[(size_t) k * HC_SL + t] = v[i];
+            xq[(size_t) k * HC_SL + t] = amax[i] == 0.0f ? 0 : (int8_t) roundf(fdiv(v[i], d));
+            if (lane == 0) xd[k * (HC_SL / 32) + warp] = d;
+            if (lane == 0 && grp == 0) red[k * (HC_SL / 32) + warp] = sq[i];
         }
     }
     __syncthreads();
@@ -135,17 +173,7 @@ __global__ void __launch_bounds__(HC_DT) k_hc_down(const HcArgs a) {
         for (int w = 0; w < HC_SL / 32; ++w) v = fadd(v, red[t * (HC_SL / 32) + w]);
         a.ssp[(size_t) t * (D / HC_SL) + s] = v;
     }
-    for (int q = warp; q < T * (HC_SL / 32); q += HC_DT / 32) {   // a warp quantises a 32-value block: float scale amax / 127
-        const int k = q / (HC_SL / 32), blk = q % (HC_SL / 32);
-        const float v = xs[(size_t) k * HC_SL + blk * 32 + lane];
-        const float amax = wmax(fabsf(v)), d = fdiv(amax, 127.0f);
-        xq[(size_t) k * HC_SL + blk * 32 + lane] = amax == 0.0f ? 0 : (int8_t) roundf(fdiv(v, d));
-        if (lane == 0) xd[k * (HC_SL / 32) + blk] = d;
-    }
-    __syncthreads();
-    const int ns = D / HC_SL;
-    (void) ns;
-#pragma unroll 1
+#pragma unroll 2
     for (int k = 0; k < T; ++k) {
         float acc = 0.f;
         if (rr < a.lr) {
@@ -153,7 +181,7 @@ __global__ void __launch_bounds__(HC_DT) k_hc_down(const HcArgs a) {
             for (int q = 0; q < NQ; ++q) {
                 const int ch = q * HC_TPR + j;
                 acc = ffma(fmul(__uint_as_float(wr[2 * NQ + q]), xd[k * (HC_SL / 32) + ch / 4]),
-                           (float) hc_dot8(make_uint2(wr[2 * q], wr[2 * q + 1]), *reinterpret_cast<const int2*>(xq + (size_t) k * HC_SL + ch * 8)), acc);
+                           hc_float(hc_dot8(make_uint2(wr[2 * q], wr[2 * q + 1]), *reinterpret_cast<const int2*>(xq + (size_t) k * HC_SL + ch * 8))), acc);
             }
         } else {
 #pragma unroll
@@ -186,10 +214,29 @@ __global__ void __launch_bounds__(256) k_hc_reduce(const HcArgs a) {
     const bool active = !inj_item || (a.w_inj && lane < a.hc);
     const int r = !active ? 0 : inj_item ? a.lr + lane : (it % nb) * 32 + lane;
     float sum = 0.f;
-    for (int cc = 0; cc < a.hc; ++cc) {
-        float p = 0.f;
-        for (int ss = 0; ss < sps; ++ss) p = fadd(p, a.part[((size_t) (cc * sps + ss) * T + k) * rows_all + r]);
-        sum = ffma(hc_rs(a, k, cc), p, sum);
+    for (int c0 = 0; c0 < a.hc; c0 += 4) {   // four streams' partials and square sums in flight together
+        float p[4] = {0.f, 0.f, 0.f, 0.f}, v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s0 = 0; s0 < sps; s0 += 8) {
+            float pv[4][8], sv[4][8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int ss = 0; ss < 8; ++ss) {
+                    const bool in = c0 + i < a.hc && s0 + ss < sps;
+                    const int at = (c0 + i) * sps + s0 + ss;
+                    pv[i][ss] = in ? a.part[((size_t) at * T + k) * rows_all + r] : 0.f;
+                    sv[i][ss] = in ? a.ssp[(size_t) k * (a.hc * sps) + at] : 0.f;
+                }
+#pragma unroll
+            for (int ss = 0; ss < 8; ++ss)
+                if (s0 + ss < sps) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p[i] = fadd(p[i], pv[i][ss]), v[i] = fadd(v[i], sv[i][ss]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c0 + i < a.hc) sum = ffma(ex_rsqrt(fadd(fdiv(v[i], (float) a.n), a.eps)), p[i], sum);
     }
     if (inj_item) {
         if (active) a.inject[k * a.hc + lane] = sum;
@@ -201,14 +248,15 @@ __global__ void __launch_bounds__(256) k_hc_reduce(const HcArgs a) {
     if (lane == 0) a.lod[k * nb + r / 32] = d;
 }
 
-// dynamic shared memory: lq [T][lr] int8, ld [T][lr / 32], rs [T][hc], ms [T][32], gs [T][hc][32]
+// dynamic shared memory: lq [T][lr] int8, ld [T][lr / 32], rs [T][hc], gt [T][hc], ms [T][32], gs [T][hc][32]
 __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
     extern __shared__ __align__(16) unsigned char hc_sm[];
     const int T = a.T, nb = a.lr / 32, hc = a.hc;
     int8_t* lq = reinterpret_cast<int8_t*>(hc_sm);
     float* ld = reinterpret_cast<float*>(lq + (size_t) T * a.lr);
     float* rs = ld + (size_t) T * nb;
-    float* ms = rs + (size_t) T * hc;
+    float* gt = rs + (size_t) T * hc;
+    float* ms = gt + (size_t) T * hc;
     float* gs = ms + (size_t) T * HC_UPC;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, b = blockIdx.x;
     const int uj = t % HC_TPU, udd = t / HC_TPU;
@@ -230,11 +278,25 @@ __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
     }
     pdl_wait();
     pdl_go();
-    if (t < T * hc) rs[t] = hc_rs(a, t / hc, t % hc);
+    // what the mix needs of R and of the ended half's rows: item e = t + 512 i is (row, stream, column), the first HC_UE
+    // items of a thread (all of them up to 16 rows of 4 streams) asked for before the dots
+    float rv[HC_UE], bv[HC_UE], wn[HC_UE];
+#pragma unroll
+    for (int i = 0; i < HC_UE; ++i) {
+        const int e = t + i * HC_UT, dc = b * HC_UPC + e % HC_UPC, cc = (e / HC_UPC) % hc, k = e / (HC_UPC * hc);
+        const bool in = e < T * hc * HC_UPC;
+        rv[i] = in ? a.R[((size_t) k * hc + cc) * a.n + dc] : 0.f;
+        bv[i] = in && a.bo ? a.bo[(size_t) k * a.n + dc] : 0.f;
+        wn[i] = in ? a.w_norm[cc * a.n + dc] : 0.f;
+    }
+    if (t < T * hc) {
+        rs[t] = hc_rs(a, t / hc, t % hc);
+        if (a.bo) gt[t] = hc_gate(a, t / hc, t % hc);
+    }
     for (int e = t; e < T * a.lr / 4; e += HC_UT) reinterpret_cast<int*>(lq)[e] = reinterpret_cast<const int*>(a.loq)[e];
     for (int e = t; e < T * nb; e += HC_UT) ld[e] = a.lod[e];
     __syncthreads();
-#pragma unroll 1
+#pragma unroll 2
     for (int k = 0; k < T; ++k) {
         const int4* xp = reinterpret_cast<const int4*>(lq + (size_t) k * a.lr + (ulive ? uj : 0) * 32);
         const int4 x0 = xp[0], x1 = xp[1];
@@ -243,7 +305,7 @@ __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
         for (int cc = 0; cc < HC_MAXS; ++cc) {
             if (cc >= hc) break;
             const uint4 w0 = wq[cc][0], w1 = wq[cc][1];
-            int sacc = __dp4a((int) w0.x, x0.x, 0);
+            int sacc = __dp4a((int) w0.x, x0.x, HC_MAGIC);
             sacc = __dp4a((int) w0.y, x0.y, sacc);
             sacc = __dp4a((int) w0.z, x0.z, sacc);
             sacc = __dp4a((int) w0.w, x0.w, sacc);
@@ -251,17 +313,22 @@ __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
             sacc = __dp4a((int) w1.y, x1.y, sacc);
             sacc = __dp4a((int) w1.z, x1.z, sacc);
             sacc = __dp4a((int) w1.w, x1.w, sacc);
-            float acc = fmul(fmul(wsc[cc], dl), (float) sacc);   // an idle lane: 0 * dl * 0
+            float acc = fmul(fmul(wsc[cc], dl), hc_float(sacc));   // an idle lane: 0 * dl * 0
             for (int o = 1; o < HC_TPU; o <<= 1) acc = fadd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
             if (uj == 0) gs[((size_t) k * hc + cc) * HC_UPC + udd] = acc;
         }
     }
     __syncthreads();
-    for (int e = t; e < T * hc * HC_UPC; e += HC_UT) {
-        const int col = e % HC_UPC, cc = (e / HC_UPC) % hc, k = e / (HC_UPC * hc), dc = b * HC_UPC + col;
-        const float rv = hc_rprime(a, k, cc, dc);
-        if (a.bo) a.R[((size_t) k * hc + cc) * a.n + dc] = rv;
-        gs[e] = fmul(ex_sigmoid(gs[e]), fmul(fmul(rv, a.w_norm[cc * a.n + dc]), rs[k * hc + cc]));
+    for (int e0 = t; e0 < T * hc * HC_UPC; e0 += HC_UE * HC_UT) {
+#pragma unroll
+        for (int i = 0; i < HC_UE; ++i) {
+            const int e = e0 + i * HC_UT, dc = b * HC_UPC + e % HC_UPC, cc = (e / HC_UPC) % hc, k = e / (HC_UPC * hc);
+            if (e >= T * hc * HC_UPC) break;
+            float* r = a.R + ((size_t) k * hc + cc) * a.n + dc;
+            if (e0 != t) rv[i] = *r, bv[i] = a.bo ? a.bo[(size_t) k * a.n + dc] : 0.f, wn[i] = a.w_norm[cc * a.n + dc];
+            if (a.bo) *r = rv[i] = ffma(bv[i], gt[k * hc + cc], rv[i]);
+            gs[e] = fmul(ex_sigmoid(gs[e]), fmul(fmul(rv[i], wn[i]), rs[k * hc + cc]));
+        }
     }
     __syncthreads();
     for (int e = t; e < T * HC_UPC; e += HC_UT) {
@@ -339,7 +406,7 @@ int fnx_hc_read(float* R, const float* bo_prev, const float* inj_prev, const flo
     if (launch_ok("hc_read down")) return 1;
     launch(0, k_hc_reduce, (T * (lr / 32) + T + 7) / 8, 256, 0, strm(st), a);
     if (launch_ok("hc_read reduce")) return 1;
-    const size_t sm3 = (size_t) T * lr + ((size_t) T * (lr / 32) + (size_t) T * hc + (size_t) T * HC_UPC + (size_t) T * hc * HC_UPC) * 4;
+    const size_t sm3 = (size_t) T * lr + ((size_t) T * (lr / 32) + (size_t) 2 * T * hc + (size_t) T * HC_UPC + (size_t) T * hc * HC_UPC) * 4;
     if (smem_optin(k_hc_up, sm3, "hc_read up")) return 1;
     launch(0, k_hc_up, n / HC_UPC, HC_UT, sm3, strm(st), a);
     return launch_ok("hc_read up");
