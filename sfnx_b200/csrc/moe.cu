@@ -21,7 +21,7 @@ namespace fnxk {
 // TMA unit's untiled copy: one instruction per group, any number of bytes in flight), a group an mbarrier, so the sums
 // over the first group run while the later ones are in flight; every block asks for the groups in an order of its own
 // (starting with group blockIdx mod groups) so that the blocks do not all pull on the same lines of the L2 at once.
-constexpr int RR_THREADS = 256, RR_ROWS = 4, RR_TG = 4;   // rows of W a block; rows of x taken together
+constexpr int RR_THREADS = 256, RR_ROWS = 4;   // rows of W a block
 
 struct RouterArgs {
     const float* W;
@@ -45,13 +45,13 @@ __device__ __forceinline__ float dot4(const float4& w, const float4& b) {
 
 __device__ void route_tail(const RouterArgs& a);
 
-template <bool SMEM>
+template <bool SMEM, int RR_TG>
 __global__ void __launch_bounds__(RR_THREADS) k_router_route(const RouterArgs a) {
     const int e = threadIdx.x, warp = e >> 5, lane = e & 31, set = warp >> 2, pair = (warp >> 1) & 1, half = warp & 1;
     const int L = a.nexp + 1, nc = a.n / 256;   // float4 chunks per lane
     extern __shared__ __align__(128) float xs_sm[];   // the window's rows of x, read once per block (when they fit)
     __shared__ float rsum[FNX_MAXT][RR_ROWS][2];
-    __shared__ __align__(8) unsigned long long xbar[(FNX_MAXT + RR_TG - 1) / RR_TG];
+    __shared__ __align__(8) unsigned long long xbar[FNX_MAXT];
     const int ngroups = (a.T + RR_TG - 1) / RR_TG, g_first = blockIdx.x % ngroups;
     if (SMEM && e == 0) {
         for (int g = 0; g < ngroups; ++g) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&xbar[g])));
@@ -142,6 +142,9 @@ __global__ void __launch_bounds__(RR_THREADS) k_router_route(const RouterArgs a)
 // min; a taken expert's key drops to 0, below every number's key.  The picks of one row are distinct experts, so a
 // 16-bit mask of rows per expert gives a pair its place inside the job (rows below it) and the job's row count, and an
 // atomic minimum gives the expert's first pair.
+// The tail is one block's work and runs once, so what it costs is latency and the fetch of its instructions: the picks
+// are a short loop that stays in the instruction cache (ranking candidates in unrolled code executed fewer steps and took
+// 3.5 us longer: 18.5 us a launch at 16 rows of 3072, now 15.1; one row 14.0, now 8.7).
 __device__ __forceinline__ unsigned logit_key(float v) {
     const unsigned b = __float_as_uint(fadd(v, 0.f));
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
@@ -155,10 +158,6 @@ __device__ void route_tail(const RouterArgs& a) {
     __shared__ unsigned rowmask[MAXE];
     __shared__ int firstpair[MAXE];
     __shared__ unsigned firstmask[PW];
-    __shared__ unsigned candk[NW][2][32];   // a warp's candidates for its two rows: keys, experts; then its picks in order
-    __shared__ int candi[NW][2][32];
-    __shared__ unsigned selk[NW][2][16];
-    __shared__ int seli[NW][2][16];
     if (e < PW) firstmask[e] = 0u;
     for (int i = e; i < a.nexp; i += RR_THREADS) rowmask[i] = 0u, firstpair[i] = P;
     // a warp takes its rows two at a time (rows t and t + NW), the two picks' instructions interleaved: each is a chain
@@ -172,123 +171,39 @@ __device__ void route_tail(const RouterArgs& a) {
             for (int i = 0; i < 16; ++i)
                 key[u][i] = (i < per && u < nu) ? logit_key(__ldcg(a.logits + (size_t) (tb + u * NW) * L + lane + 32 * i)) : 0u;
         float mine[2] = {0.f, 0.f}, top0[2] = {0.f, 0.f};   // lane k keeps pick k's logit
-        // The k-th largest of the 32 lanes' maxima is a lower bound of the k-th largest key (k keys reach it), so the
-        // picks are among the keys that reach it: a handful, ranked by counting (a greater key, or an equal key of a
-        // lower expert, comes first).  Many equal keys can make the candidates more than a warp holds: then pick by pick.
-        unsigned lm[2], hitm[2] = {0u, 0u};
-        int rk[2] = {0, 0}, cnt[2], pre[2], total[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            lm[u] = key[u][0];
-#pragma unroll
-            for (int i = 1; i < 16; ++i) lm[u] = max(lm[u], key[u][i]);
-        }
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
+        int pick[2] = {0, 0};                                // and its expert
+#pragma unroll 1
+        for (int k = 0; k < a.topk; ++k) {
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const unsigned o = __shfl_sync(0xffffffffu, lm[u], j);
-                rk[u] += (o > lm[u]) | ((o == lm[u]) & (j < lane));
-            }
+                unsigned m = 0u;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const unsigned bound = __reduce_max_sync(0xffffffffu, rk[u] == a.topk - 1 ? lm[u] : 0u);
+                for (int i = 0; i < 16; ++i) m = max(m, key[u][i]);
+                const unsigned M = __reduce_max_sync(0xffffffffu, m);
+                unsigned c = 0xffffffffu;   // this lane's lowest expert with the largest key
 #pragma unroll
-            for (int i = 0; i < 16; ++i) hitm[u] |= (unsigned) (i < per && u < nu && key[u][i] >= bound) << i;
-            cnt[u] = pre[u] = __popc(hitm[u]);   // pre: inclusive scan over the lanes
-        }
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1)
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int o = __shfl_up_sync(0xffffffffu, pre[u], d);
-                if (lane >= d) pre[u] += o;
-            }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) total[u] = __shfl_sync(0xffffffffu, pre[u], 31);
-        const bool fast = a.topk <= 32 && total[0] <= 32 && total[1] <= 32;   // warp-uniform
-        if (fast) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                int o = pre[u] - cnt[u];
+                for (int i = 15; i >= 0; --i)
+                    if (key[u][i] == M) c = (unsigned) (lane + 32 * i);
+                const unsigned bi = __reduce_min_sync(0xffffffffu, c);
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                    if ((hitm[u] >> i) & 1u) {
-                        candk[warp][u][o] = key[u][i];
-                        candi[warp][u][o] = lane + 32 * i;
-                        ++o;
-                    }
-            }
-            __syncwarp();
-            unsigned myk[2];
-            int myi[2], r[2] = {0, 0};
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                myk[u] = lane < total[u] ? candk[warp][u][lane] : 0u;
-                myi[u] = lane < total[u] ? candi[warp][u][lane] : 0x7fffffff;
-            }
-            const int tmax = max(total[0], total[1]);
-            for (int j = 0; j < tmax; ++j)
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const unsigned ok = j < total[u] ? candk[warp][u][j] : 0u;
-                    const int oi = j < total[u] ? candi[warp][u][j] : 0x7fffffff;
-                    r[u] += (ok > myk[u]) | ((ok == myk[u]) & (oi < myi[u]));
-                }
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-                if (lane < total[u] && r[u] < a.topk) selk[warp][u][r[u]] = myk[u], seli[warp][u][r[u]] = myi[u];
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (u >= nu) break;
-                const int t = tb + u * NW;
-                top0[u] = key_logit(selk[warp][u][0]);
-                if (lane < a.topk) {
-                    const int bi = seli[warp][u][lane];
-                    mine[u] = key_logit(selk[warp][u][lane]);
-                    a.topi[t * a.topk + lane] = bi;
-                    ex[t * a.topk + lane] = bi;
-                }
-            }
-            __syncwarp();
-        } else {
-            for (int u = 0; u < nu; ++u) {
-                const int t = tb + u * NW;
-                unsigned kk[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) kk[i] = u ? key[1][i] : key[0][i];
-                float mn = 0.f, tp = 0.f;
-                for (int k = 0; k < a.topk; ++k) {
-                    unsigned m = kk[0];
-#pragma unroll
-                    for (int i = 1; i < 16; ++i) m = max(m, kk[i]);
-                    const unsigned M = __reduce_max_sync(0xffffffffu, m);
-                    unsigned hit = 0u;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) hit |= (unsigned) (kk[i] == M) << i;
-                    const unsigned cand = hit ? (unsigned) (lane + 32 * (__ffs(hit) - 1)) : 0xffffffffu;
-                    const int bi = (int) __reduce_min_sync(0xffffffffu, cand);
-                    if ((bi & 31) == lane) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (i == (bi >> 5)) kk[i] = 0u;
-                    }
-                    const float bv = key_logit(M);
-                    if (k == 0) tp = bv;
-                    if (lane == k) {
-                        mn = bv;
-                        a.topi[t * a.topk + k] = bi;
-                        ex[t * a.topk + k] = bi;
-                    }
-                }
-                if (u) mine[1] = mn, top0[1] = tp;
-                else mine[0] = mn, top0[0] = tp;
+                    if (bi == (unsigned) (lane + 32 * i)) key[u][i] = 0u;
+                const float bv = key_logit(M);
+                if (k == 0) top0[u] = bv;
+                if (lane == k) mine[u] = bv, pick[u] = (int) bi;
             }
         }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (u < nu && lane < a.topk) {
+                const int t = tb + u * NW;
+                a.topi[t * a.topk + lane] = pick[u];
+                ex[t * a.topk + lane] = pick[u];
+            }
         float ek[2], z[2] = {0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < 2; ++u) ek[u] = ex_expf(fsub(mine[u], top0[u]));
+#pragma unroll 1
         for (int k = 0; k < a.topk; ++k)
 #pragma unroll
             for (int u = 0; u < 2; ++u) z[u] = fadd(z[u], __shfl_sync(0xffffffffu, ek[u], k));
@@ -309,6 +224,7 @@ __device__ void route_tail(const RouterArgs& a) {
     for (int p = e; p < P; p += RR_THREADS) {
         const int x = ex[p], fp = firstpair[x], t = p / a.topk;
         int j = 0;   // jobs that start before this pair's expert's first pair
+#pragma unroll 1
         for (int k = 0; k < words; ++k) {
             if (32 * k + 31 < fp) j += __popc(firstmask[k]);
             else if (32 * k <= fp) j += __popc(firstmask[k] & ((1u << (fp - 32 * k)) - 1u));
@@ -833,12 +749,22 @@ int fnx_router_route(const float* W, const float* x, float* logits, int T, int n
     const bool fits = xbytes <= 200 * 1024 && ((uintptr_t) x % 16) == 0;
     int grid = (nexp + 1 + RR_ROWS - 1) / RR_ROWS;
     if (grid > 148) grid = 148;
-    if (fits) {
-        if (smem_optin(k_router_route<true>, xbytes, "router_route")) return 1;
-        launch(2, k_router_route<true>, grid, RR_THREADS, xbytes, strm(st), a);
-    } else {
-        launch(2, k_router_route<false>, grid, RR_THREADS, 0, strm(st), a);
+    // rows of x taken together: no more than the window has (one row takes a quarter of the steps, and of the code, of four)
+#define RR_LAUNCH(TG)                                                                         \
+    if (fits) {                                                                               \
+        if (smem_optin(k_router_route<true, TG>, xbytes, "router_route")) return 1;           \
+        launch(2, k_router_route<true, TG>, grid, RR_THREADS, xbytes, strm(st), a);           \
+    } else {                                                                                  \
+        launch(2, k_router_route<false, TG>, grid, RR_THREADS, 0, strm(st), a);               \
     }
+    if (T == 1) {
+        RR_LAUNCH(1)
+    } else if (T == 2) {
+        RR_LAUNCH(2)
+    } else {
+        RR_LAUNCH(4)
+    }
+#undef RR_LAUNCH
     return launch_ok("router_route");
 }
 
@@ -852,7 +778,7 @@ int fnx_moe_gate_up(const FnxExperts* A, const FnxJob* jobs, const int* njobs, i
         // blocks of 128 rows with direct 16-byte loads one step ahead (measured faster than staging the weights through
         // shared memory, by cp.async rings or bulk copies: there every operand crosses the shared-memory pipe)
         // rows of 128 a block, of 64 where an expert has few rows or a window so few jobs that the longer blocks would not
-        // give every multiprocessor one: the launch is over sooner (one row's ten jobs at 1536 x 3072: 12.0 us, TIMEB us)
+        // give every multiprocessor one: the launch is over sooner (one row's ten jobs at 1536 x 3072: 12.0 us, now 9.6)
         const int blocks128 = (nrows + GU_THREADS / 2 - 1) / (GU_THREADS / 2) * njobs_max;
         const int R = (nrows <= 512 || blocks128 < 148) && (n / 512) % 2 == 0 ? 2 : 4, rpb = GU_THREADS / 8 * R;   // the step count must stay even
         const dim3 grid((nrows + rpb - 1) / rpb, njobs_max);
