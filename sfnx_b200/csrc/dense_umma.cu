@@ -9,10 +9,10 @@
 //   warp 16   the TMA unit's driver: for every 128 bytes of K (four blocks) one cp.async.bulk.tensor load of the 128 x 128
 //             byte weight tile into a 128-byte-swizzled stage (six stages), and per tile one load of its f16 block scales;
 //             it starts before the kernel ahead in the stream has finished (weights depend on nothing in the window)
-//   warp 17   issues the four MMAs of a stage, each into its own 16 columns of one of eight 64-column groups of tensor
-//             memory; tcgen05.commit hands the stage back to the TMA warp and the group to the epilogue
+//   warp 17   issues the four MMAs of a stage, each into its own 16 columns of one of four 128-column groups of tensor
+//             memory; tcgen05.commit hands the stage back to the TMA warp and, every second stage, the group to the epilogue
 //   warps 0-15  the epilogue: warp w reads rows 32 (w % 4) .. + 31 (its quarter of tensor memory) and window rows
-//             4 (w / 4) .. + 3: tcgen05.ld, the integer dots to float by the 1.5 * 2^23 offset (no convert instruction),
+//             4 (w / 4) .. + 3 (the warps of rows that the window does not have leave at once): tcgen05.ld, the integer dots to float by the 1.5 * 2^23 offset (no convert instruction),
 //             scale by fl(dw da) and add - sixteen warps so that the CUDA-core work of a 4 KB block step (128 rows x 16
 //             values) stays well under the time HBM needs to deliver the step.
 // The window's activations (int8 plane as the MMAs' B operand, 16 rows x K, and their float scales) are staged once per
@@ -29,7 +29,7 @@
 
 namespace fnxk {
 
-constexpr int DU_M = 128, DU_KC = 128, DU_STAGES = 6, DU_SLOTS = 8, DU_EPI = 16, DU_THREADS = (DU_EPI + 2) * 32, DU_MAXCOLS = 3072;
+constexpr int DU_M = 128, DU_KC = 128, DU_STAGES = 6, DU_SLOTS = 4, DU_EPI = 16, DU_THREADS = (DU_EPI + 2) * 32, DU_MAXCOLS = 3072;
 constexpr int DU_ABYTES = DU_M * DU_KC, DU_BCHUNK = 16 * DU_KC, DU_MAGIC = 0x4B400000;
 
 struct DuMaps {
@@ -38,7 +38,7 @@ struct DuMaps {
 struct DuArgs {
     int nseg, rows[3], tile_end[3], stride[3];
     float* out[3];
-    int cols, T, ntiles;
+    int cols, T, ntiles, H;   // H: weight rows a tile, up to DU_M
     const uint8_t* yq;
     unsigned* fault;
 };
@@ -89,17 +89,18 @@ struct DuTile {
 };
 __device__ __forceinline__ DuTile du_tile(const DuArgs& a, int tile) {
     const int seg = tile < a.tile_end[0] ? 0 : tile < a.tile_end[1] ? 1 : 2;
-    return DuTile{seg, (tile - (seg == 0 ? 0 : seg == 1 ? a.tile_end[0] : a.tile_end[1])) * DU_M};
+    return DuTile{seg, (tile - (seg == 0 ? 0 : seg == 1 ? a.tile_end[0] : a.tile_end[1])) * a.H};
 }
 
 __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constant__ DuMaps maps, const DuArgs a) {
     extern __shared__ unsigned char du_smem[];
     unsigned char* base = du_smem + ((1024u - (um_s32(du_smem) & 1023u)) & 1023u);   // swizzled tiles start on 1024-byte boundaries
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = a.cols / 32, nkc = a.cols / DU_KC;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = a.cols / 32, nkc = a.cols / DU_KC, ngrp = (a.T + 3) / 4;
+    const int nd = (nb + 15) / 16;   // boxes of 16 block scales
     unsigned char* a_st = base;                                                // [DU_STAGES][128 rows][128 bytes], swizzled
     unsigned char* b_op = a_st + (size_t) DU_STAGES * DU_ABYTES;               // [nkc][16 rows][128 bytes], swizzled
-    uint16_t* dw_s = reinterpret_cast<uint16_t*>(b_op + (size_t) nkc * DU_BCHUNK);   // [2][128][nb] f16 block scales of a tile
-    float* da_s = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(dw_s) + (size_t) 2 * DU_M * nb * 2);   // [nb][16]
+    uint16_t* dw_s = reinterpret_cast<uint16_t*>(b_op + (size_t) nkc * DU_BCHUNK);   // [2][nd][128][16] f16 block scales of a tile, swizzled in 32 bytes
+    float* da_s = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(dw_s) + (size_t) 2 * DU_M * nd * 32);   // [nb][16]
     __shared__ __align__(8) unsigned long long full_a[DU_STAGES], empty_a[DU_STAGES], tm_full[DU_SLOTS], tm_empty[DU_SLOTS], dw_full[2], dw_empty[2];
     __shared__ unsigned tmem_base;
     if (tid == 0) {
@@ -109,15 +110,15 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
         }
         for (int s = 0; s < DU_SLOTS; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&tm_full[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&tm_empty[s])), "r"(DU_EPI));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&tm_empty[s])), "r"(4 * ngrp));
         }
         for (int s = 0; s < 2; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&dw_full[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&dw_empty[s])), "r"(DU_EPI));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&dw_empty[s])), "r"(4 * ngrp));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == DU_EPI + 1) {   // all 512 columns of tensor memory: eight groups of 4 x 16
+    if (warp == DU_EPI + 1) {   // all 512 columns of tensor memory: four groups of 2 x 4 x 16
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(um_s32(&tmem_base)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -135,12 +136,12 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                 const CUtensorMap* mw = &maps.w[t.seg];
                 const CUtensorMap* md = &maps.d[t.seg];
                 if (nt >= 2 && alive) alive = um_wait(&dw_empty[tp], (unsigned) ((nt / 2 - 1) & 1), a.fault);
-                um_expect_tx(&dw_full[tp], (unsigned) (DU_M * nb * 2));
-                um_tma2d(um_s32(dw_s + (size_t) tp * DU_M * nb), md, 0, t.row0, &dw_full[tp]);
+                um_expect_tx(&dw_full[tp], (unsigned) (a.H * nd * 32));
+                for (int i = 0; i < nd; ++i) um_tma2d(um_s32(dw_s) + (tp * nd + i) * DU_M * 32, md, 16 * i, t.row0, &dw_full[tp]);
                 for (int kc = 0; kc < nkc; ++kc, ++c) {
                     const int s = c % DU_STAGES;
                     if (c >= DU_STAGES && alive) alive = um_wait(&empty_a[s], (unsigned) ((c / DU_STAGES - 1) & 1), a.fault);
-                    um_expect_tx(&full_a[s], DU_ABYTES);
+                    um_expect_tx(&full_a[s], (unsigned) (a.H * DU_KC));
                     um_tma2d(a_s32 + s * DU_ABYTES, mw, kc * DU_KC, t.row0, &full_a[s]);
                 }
             }
@@ -173,20 +174,20 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
             int c = 0;
             for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
                 for (int kc = 0; kc < nkc; ++kc, ++c) {
-                    const int s = c % DU_STAGES, slot = c % DU_SLOTS;
+                    const int s = c % DU_STAGES, slot = (c >> 1) % DU_SLOTS, use = (c >> 1) / DU_SLOTS;
                     if (alive) alive = um_wait(&full_a[s], (unsigned) ((c / DU_STAGES) & 1), a.fault);
-                    if (c >= DU_SLOTS && alive) alive = um_wait(&tm_empty[slot], (unsigned) ((c / DU_SLOTS - 1) & 1), a.fault);
+                    if (!(c & 1) && use && alive) alive = um_wait(&tm_empty[slot], (unsigned) ((use - 1) & 1), a.fault);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (lane == 0) {
                         const unsigned long long da = um_desc(a_s32 + s * DU_ABYTES), db = um_desc(b_s32 + kc * DU_BCHUNK);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) du_mma_i8(tmem_base + (unsigned) (slot * 64 + 16 * j), da + 2 * j, db + 2 * j, idesc);
+                        for (int j = 0; j < 4; ++j) du_mma_i8(tmem_base + (unsigned) (slot * 128 + (c & 1) * 64 + 16 * j), da + 2 * j, db + 2 * j, idesc);
                         du_commit(&empty_a[s]);
-                        du_commit(&tm_full[slot]);
+                        if (c & 1) du_commit(&tm_full[slot]);   // tracks every MMA before it; the stages of a tile are even in number
                     }
                     __syncwarp();
                 }
-        } else {
+        } else if ((warp >> 2) < ngrp) {
             // ---- the epilogue warps
             const int q = warp & 3, g = warp >> 2, r_in = 32 * q + lane;
             int c = 0, tp = 0, nt = 0;
@@ -194,20 +195,22 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                 const DuTile t = du_tile(a, tile);
                 if (alive) alive = um_wait(&dw_full[tp], (unsigned) ((nt / 2) & 1), a.fault);
                 alive = __all_sync(0xffffffffu, alive);
-                const uint16_t* dwr = dw_s + ((size_t) tp * DU_M + r_in) * nb;
+                // eight block scales (two stages' worth) in one 16-byte read, the rows' pieces swizzled over the banks
+                const unsigned char* dwr = reinterpret_cast<const unsigned char*>(dw_s) + (size_t) tp * nd * DU_M * 32 + r_in * 32;
+                const int dsw = (r_in >> 2) & 1;
                 du_f32x2 acc01 = 0ull, acc23 = 0ull;   // window rows 4 g, + 1 and + 2, + 3 of this thread's weight row
                 const du_f32x2 unmagic = du_pack(-12582912.0f, -12582912.0f);
                 const float* dap = da_s + 4 * g;
-#pragma unroll 2
-                for (int kc = 0; kc < nkc; ++kc, ++c) {
+#pragma unroll 1
+                for (int kc = 0; kc < nkc; kc += 2, ++c) {   // two stages: eight blocks
                     const int slot = c % DU_SLOTS;
-                    const uint2 dwh = *reinterpret_cast<const uint2*>(dwr + 4 * kc);   // this stage's four block scales
+                    const uint4 dwh = *reinterpret_cast<const uint4*>(dwr + (size_t) (kc >> 2) * DU_M * 32 + ((((kc >> 1) & 1) ^ dsw) << 4));
                     if (alive) alive = um_wait(&tm_full[slot], (unsigned) ((c / DU_SLOTS) & 1), a.fault);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    unsigned v[16];
-                    const unsigned ta = tmem_base + ((unsigned) (32 * q) << 16) + (unsigned) (slot * 64 + 4 * g);
+                    unsigned v[32];
+                    const unsigned ta = tmem_base + ((unsigned) (32 * q) << 16) + (unsigned) (slot * 128 + 4 * g);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 8; ++j)
                         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                                      : "=r"(v[4 * j]), "=r"(v[4 * j + 1]), "=r"(v[4 * j + 2]), "=r"(v[4 * j + 3])
                                      : "r"(ta + 16 * j));
@@ -215,9 +218,9 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) du_arrive(&tm_empty[slot]);   // the group may be overwritten: its values are in registers
-                    const unsigned dww[2] = {dwh.x, dwh.y};
+                    const unsigned dww[4] = {dwh.x, dwh.y, dwh.z, dwh.w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < 8; ++j) {
                         const float dw = h2f((uint16_t) (j & 1 ? dww[j >> 1] >> 16 : dww[j >> 1] & 0xffff));
                         const du_f32x2 dw2 = du_pack(dw, dw);
                         const ulonglong2 da4 = *reinterpret_cast<const ulonglong2*>(dap + (size_t) (4 * kc + j) * 16);
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                 float* out = seg == 0 ? a.out[0] : seg == 1 ? a.out[1] : a.out[2];
                 const int stride = seg == 0 ? a.stride[0] : seg == 1 ? a.stride[1] : a.stride[2];
                 const int rows = seg == 0 ? a.rows[0] : seg == 1 ? a.rows[1] : a.rows[2];
-                if (row < rows) {
+                if (row < rows && r_in < a.H) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (4 * g + i < a.T) out[(size_t) (4 * g + i) * stride + row] = acc[i];
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
 // ---- host side: tensor maps over this GPU's own memory (plain loads, no multicast)
 size_t q8s_umma_smem(int cols) {
     const int nb = cols / 32, nkc = cols / DU_KC;
-    return (size_t) DU_STAGES * DU_ABYTES + (size_t) nkc * DU_BCHUNK + (size_t) 2 * DU_M * nb * 2 + (size_t) nb * 16 * 4 + 1024;
+    return (size_t) DU_STAGES * DU_ABYTES + (size_t) nkc * DU_BCHUNK + (size_t) 2 * DU_M * ((nb + 15) / 16) * 32 + (size_t) nb * 16 * 4 + 1024;
 }
 
 // the tensor-core dense kernel over 1..3 matrices of `cols` columns; -1 when the shape is not its (the caller uses the
@@ -270,32 +273,44 @@ int q8s_umma_launch(const FnxQ8S* w, const int* rows, float* const* out, const i
     UmEncode enc = um_encoder();
     unsigned* fault = device_fault_word();
     if (!enc || !fault) return fail("%s: no tensor-map encoder or fault word", what);
-    DuMaps maps;
-    DuArgs a{};
-    a.nseg = nseg, a.cols = cols, a.T = T, a.yq = (const uint8_t*) yq, a.fault = fault;
-    int nt = 0;
-    for (int s = 0; s < 3; ++s) {
-        const int k = s < nseg ? s : nseg - 1;
-        const cuuint64_t gd_w[2] = {(cuuint64_t) cols, (cuuint64_t) rows[k]}, gs_w[1] = {(cuuint64_t) cols};
-        const cuuint32_t bx_w[2] = {DU_KC, DU_M}, es[2] = {1, 1};
-        const cuuint64_t gd_d[2] = {(cuuint64_t) (cols / 32), (cuuint64_t) rows[k]}, gs_d[1] = {(cuuint64_t) (cols / 32) * 2};
-        const cuuint32_t bx_d[2] = {(cuuint32_t) (cols / 32), DU_M};
-        if (enc(&maps.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*) w[k].q, gd_w, gs_w, bx_w, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
-            enc(&maps.d[s], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*) w[k].d, gd_d, gs_d, bx_d, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return fail("%s: tensor map of a %d x %d matrix refused", what, rows[k], cols);
-        a.rows[s] = rows[k], a.stride[s] = out_stride[k], a.out[s] = out[k];
-        if (s < nseg) nt += (rows[s] + DU_M - 1) / DU_M;
-        a.tile_end[s] = nt;
-    }
-    a.ntiles = nt;
     static int nsm = 0;
     if (!nsm) {
         int dev = 0;
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 148;
     }
+    // Rows a tile: a tile's time hardly depends on its rows as long as it is one, so the smallest height that takes no more
+    // rounds of the GPU than 128 does spreads the bytes evenly over the multiprocessors (a head of 151 936 rows: 9 rounds
+    // of 115 rows, not 8 of 128 and one of 3 tiles; 14 336 rows of wq|wk|wv: 148 tiles of 98, not 112 of 128).
+    auto tiles_of = [&](int h) {
+        long t = 0;
+        for (int s = 0; s < nseg; ++s) t += (rows[s] + h - 1) / h;
+        return t;
+    };
+    const long rounds = (tiles_of(DU_M) + nsm - 1) / nsm;
+    int H = DU_M;
+    while (H > 64 && (tiles_of(H - 1) + nsm - 1) / nsm <= rounds) --H;
+    DuMaps maps;
+    DuArgs a{};
+    a.H = H;
+    a.nseg = nseg, a.cols = cols, a.T = T, a.yq = (const uint8_t*) yq, a.fault = fault;
+    int nt = 0;
+    for (int s = 0; s < 3; ++s) {
+        const int k = s < nseg ? s : nseg - 1;
+        const cuuint64_t gd_w[2] = {(cuuint64_t) cols, (cuuint64_t) rows[k]}, gs_w[1] = {(cuuint64_t) cols};
+        const cuuint32_t bx_w[2] = {DU_KC, (cuuint32_t) H}, es[2] = {1, 1};
+        const cuuint64_t gd_d[2] = {(cuuint64_t) (cols / 32), (cuuint64_t) rows[k]}, gs_d[1] = {(cuuint64_t) (cols / 32) * 2};
+        const cuuint32_t bx_d[2] = {16, (cuuint32_t) H};
+        if (enc(&maps.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*) w[k].q, gd_w, gs_w, bx_w, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+            enc(&maps.d[s], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*) w[k].d, gd_d, gs_d, bx_d, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
+                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("%s: tensor map of a %d x %d matrix refused", what, rows[k], cols);
+        a.rows[s] = rows[k], a.stride[s] = out_stride[k], a.out[s] = out[k];
+        if (s < nseg) nt += (rows[s] + H - 1) / H;
+        a.tile_end[s] = nt;
+    }
+    a.ntiles = nt;
     const size_t sm = q8s_umma_smem(cols);
     if (smem_optin(k_q8s_umma, sm, what)) return 1;
     launch(1, k_q8s_umma, std::min(nsm, nt), DU_THREADS, sm, st, maps, a);

@@ -55,7 +55,7 @@ def test_q8s_gemv(rows, cols, T):
     assert np.array_equal(G.host(out).view(np.uint32), ref.view(np.uint32))
 
 
-@pytest.mark.parametrize("rows,cols,T", [(16384, 3072, 16), (8200, 1024, 5), (40000, 2560, 1), (9000, 256, 16)])
+@pytest.mark.parametrize("rows,cols,T", [(16384, 3072, 16), (8200, 1024, 5), (40000, 2560, 1), (9000, 256, 16), (39001, 768, 4), (19000, 512, 9)])
 def test_q8s_gemv_blocks_tensor_cores(rows, cols, T):
     """The tcgen05 dense kernel: bit-equal to the oracle's statement of its order of sums (blocks in ascending order), equal
     to the reference-order product to fp32 rounding of the sum, over ragged row counts (a last tile past the matrix), one
