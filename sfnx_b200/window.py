@@ -481,7 +481,7 @@ class WindowRunner:
         self.h_jobs = torch.zeros(64 * self.job_bytes, dtype=torch.uint8).pin_memory()   # a ring of job tables
         self.commits = 0
         self.launches = 0
-        self.graph = None
+        self.graph = self.graph_io = None
         # a side stream for the window's independent branches (the library forks and joins with these events)
         self.side = torch.cuda.Stream() if overlap else None
         self.ev_fork, self.ev_join = torch.cuda.Event(), torch.cuda.Event()
@@ -496,6 +496,13 @@ class WindowRunner:
                 with torch.cuda.graph(g, stream=self.stream):
                     self._enqueue()
                 self.graph = g
+                if self.dist is None:   # the host calls' window: the upload and the read-back are nodes of the graph, one launch in all
+                    g = torch.cuda.CUDAGraph()
+                    with torch.cuda.graph(g, stream=self.stream):
+                        self._upload()
+                        self._enqueue()
+                        self._read_back()
+                    self.graph_io = g
         torch.cuda.synchronize()
 
     def _make_ring(self, count):
@@ -589,6 +596,15 @@ class WindowRunner:
                 self.dist.all_gather_into_tensor(self.all_ci.view(-1), self.cand_i.view(-1), group=self.group)
         self.d_out[-1:].copy_(self.err)
 
+    def _upload(self):
+        self.d_in.copy_(self.h_in, non_blocking=True)
+
+    def _read_back(self):
+        self.h_out.copy_(self.d_out, non_blocking=True)
+        if self.sampled:
+            self.h_cv.copy_(self.all_cv, non_blocking=True)
+            self.h_ci.copy_(self.all_ci, non_blocking=True)
+
     def launch(self):
         """Enqueues one window on the runner's stream (the caller has set ids and ctl)."""
         with torch.cuda.stream(self.stream):
@@ -611,9 +627,12 @@ class WindowRunner:
     def _run(self):
         """Uploads the host's ids and control words, runs the window, reads the result back and merges it."""
         with torch.cuda.stream(self.stream):
-            self.d_in.copy_(self.h_in, non_blocking=True)
-            self.launch()
-            self.h_out.copy_(self.d_out, non_blocking=True)
+            if self.graph_io is not None:
+                self.graph_io.replay()
+            else:
+                self._upload()
+                self.launch()
+                self._read_back()
         self.stream.synchronize()
         err = int(self.h_err[0])
         if err != 0:
@@ -638,8 +657,9 @@ class WindowRunner:
             tok = self.window([token], pos0 + i, tag)[0]
             out.append(tok)
             token = tok
-            with torch.cuda.stream(self.stream):
-                self.src[0].copy_(streams)
+            if i + 1 < k:
+                with torch.cuda.stream(self.stream):
+                    self.src[0].copy_(streams)
         return out
 
     def window_lanes(self, rows, pos, tags):
@@ -677,11 +697,7 @@ class WindowRunner:
         number); the caller commits that many rows."""
         assert self.sampled, "build the runner with sampled=True"
         T, lib = self.T, L.load()
-        self.window(rows, pos0, tag)
-        with torch.cuda.stream(self.stream):
-            self.h_cv.copy_(self.all_cv, non_blocking=True)
-            self.h_ci.copy_(self.all_ci, non_blocking=True)
-        self.stream.synchronize()
+        self.window(rows, pos0, tag)   # reads the candidates back with the result
         mv = (C.c_float * (T * L.TOPK_N))()
         mi = (C.c_int * (T * L.TOPK_N))()
         if lib.fnx_top_merge(self.h_cv.data_ptr(), self.h_ci.data_ptr(), self.stack.ncard, T, mv, mi) != 0:
@@ -709,7 +725,7 @@ class WindowRunner:
         """Releases what must go before the process group does: the captured graph (its NCCL nodes hold the communicator)
         and the peer-mapped buffers of the sum across GPUs."""
         torch.cuda.synchronize()
-        self.graph = None
+        self.graph = self.graph_io = None
         self.ring = None
         self.ring_keep = None
         torch.cuda.synchronize()
