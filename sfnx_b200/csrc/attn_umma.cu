@@ -116,7 +116,7 @@ constexpr int A3_NBUF = 3, A3_PBYTES = A3_QROWS * 128, A3_PAD = 4096;   // the p
 template <bool TMA>
 __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant__ AuMaps maps, const AuArgs a) {
     constexpr int HD = AU_HD;
-    const int split = blockIdx.x, kvl = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x;
+    const int split = blockIdx.x, kvl = blockIdx.y, tid = threadIdx.x, warp = (int) um_uniform(tid >> 5), lane = tid & 31, nthreads = blockDim.x;
     const int qpk = a.nq / a.nkv, M = a.T * qpk;
     extern __shared__ __align__(1024) unsigned char au_smem[];
     unsigned char* Qhi = au_smem + ((1024u - (um_s32(au_smem) & 1023u)) & 1023u);
@@ -221,8 +221,9 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     const float rs = 1.0f / sqrtf((float) HD);
     const unsigned idesc_s = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);               // S: N 64, both operands K-major
     const unsigned idesc_o = (1u << 4) | (1u << 16) | ((256u >> 3) << 17) | ((128u >> 4) << 24);   // O: N 256, B MN-major
+    unsigned tm = 0;   // the tensor memory's base, once it is allocated
     auto issue_scores = [&](int c) {
-        const unsigned tb = tmem_base + AU2_COL_S + (c & 1) * A3_CH;
+        const unsigned tb = tm + AU2_COL_S + (c & 1) * A3_CH;
         const unsigned long long dk = um_desc(um_s32(KVst + (size_t) (c % A3_NBUF) * A3_KBYTES));
         const unsigned long long dh = um_desc(um_s32(Qhi)), dl = um_desc(um_s32(Qlo));
 #pragma unroll
@@ -240,8 +241,8 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         const unsigned long long dph = um_desc(um_s32(Pst)), dpl = um_desc(um_s32(Pst + A3_PBYTES));
 #pragma unroll
         for (int ks = 0; ks < A3_CH / 16; ++ks) {
-            um_mma(tmem_base, dph + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, c | ks);
-            um_mma(tmem_base, dpl + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, 1u);
+            um_mma(tm, dph + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, c | ks);
+            um_mma(tm, dpl + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, 1u);
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&mbar_o)) : "memory");
     };
@@ -253,10 +254,12 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     };
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     sync_all();
-    const bool issuer = tid == 3 * 32;   // warp 3, lane 0
+    tm = um_uniform(tmem_base);
+    const bool issuer = warp == 3;   // one lane of it
     if (issuer) {
         if (TMA) um_wait(&qbar, 0u, a.fault), um_wait(&kvbar[0], 0u, a.fault);   // the queries and K(0) have landed
-        issue_scores(0);
+        if (um_elect()) issue_scores(0);
+        __syncwarp();
     }
     bool alive = true;   // false after a wait ran out
     auto copier_wait = [&](unsigned long long* bar, unsigned parity) {   // the copying warp alone waits for a set of MMAs
@@ -275,7 +278,8 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         const int buf = i & 1;
         if (issuer && i + 1 < nc) {   // the next chunk's scores while this chunk's are used
             if (TMA) um_wait(&kvbar[(i + 1) % A3_NBUF], 0u, a.fault);   // K(i + 1) has landed
-            issue_scores(i + 1);
+            if (um_elect()) issue_scores(i + 1);
+            __syncwarp();
         }
         float sacc[8][4];
 #pragma unroll
@@ -401,7 +405,10 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
                 *reinterpret_cast<uint4*>(KVst + (size_t) (i % A3_NBUF) * A3_KBYTES + (lane >> 3) * A3_KBLK + row * 128 + (lane & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
         }
         sync_all();
-        if (issuer) issue_output(i);
+        if (issuer) {
+            if (um_elect()) issue_output(i);
+            __syncwarp();
+        }
     }
     // ---- this split's partial: the accumulator out of tensor memory, m_ref, z per row
     {

@@ -95,7 +95,7 @@ __device__ __forceinline__ DuTile du_tile(const DuArgs& a, int tile) {
 __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constant__ DuMaps maps, const DuArgs a) {
     extern __shared__ unsigned char du_smem[];
     unsigned char* base = du_smem + ((1024u - (um_s32(du_smem) & 1023u)) & 1023u);   // swizzled tiles start on 1024-byte boundaries
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = a.cols / 32, nkc = a.cols / DU_KC, ngrp = (a.T + 3) / 4;
+    const int tid = threadIdx.x, warp = (int) um_uniform(tid >> 5), lane = tid & 31, nb = a.cols / 32, nkc = a.cols / DU_KC, ngrp = (a.T + 3) / 4;
     const int nd = (nb + 15) / 16;   // boxes of 16 block scales
     unsigned char* a_st = base;                                                // [DU_STAGES][128 rows][128 bytes], swizzled
     unsigned char* b_op = a_st + (size_t) DU_STAGES * DU_ABYTES;               // [nkc][16 rows][128 bytes], swizzled
@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
         asm volatile("bar.sync 1, %0;" ::"n"(DU_THREADS - 32) : "memory");
         if (warp == DU_EPI + 1) {
             // ---- the issuing warp
+            const unsigned tm = um_uniform(tmem_base);
             const unsigned idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);   // D s32, A and B s8 K-major, N 16, M 128
             int c = 0;
             for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
@@ -178,10 +179,10 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                     if (alive) alive = um_wait(&full_a[s], (unsigned) ((c / DU_STAGES) & 1), a.fault);
                     if (!(c & 1) && use && alive) alive = um_wait(&tm_empty[slot], (unsigned) ((use - 1) & 1), a.fault);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
+                    if (um_elect()) {
                         const unsigned long long da = um_desc(a_s32 + s * DU_ABYTES), db = um_desc(b_s32 + kc * DU_BCHUNK);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) du_mma_i8(tmem_base + (unsigned) (slot * 128 + (c & 1) * 64 + 16 * j), da + 2 * j, db + 2 * j, idesc);
+                        for (int j = 0; j < 4; ++j) du_mma_i8(tm + (unsigned) (slot * 128 + (c & 1) * 64 + 16 * j), da + 2 * j, db + 2 * j, idesc);
                         du_commit(&empty_a[s]);
                         if (c & 1) du_commit(&tm_full[slot]);   // tracks every MMA before it; the stages of a tile are even in number
                     }

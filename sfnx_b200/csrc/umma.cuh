@@ -26,6 +26,16 @@ __device__ __forceinline__ void um_mma(unsigned tmem, unsigned long long da, uns
                  : "memory");
 }
 
+// One lane of a converged warp, the same one each time.  The branch it guards stays uniform for the compiler, so that
+// descriptors stay in uniform registers: under `lane == 0` each tcgen05.mma spent about 110 cycles moving them there.
+__device__ __forceinline__ bool um_elect() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// a warp-uniform value, known to be one
+__device__ __forceinline__ unsigned um_uniform(unsigned v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // Waits for the phase of `bar` with this parity; gives up after 2^22 polls, sets bit 8 of *fault and returns false (the
 // caller goes on with what it has: no wait in these kernels is unbounded).
 __device__ __forceinline__ bool um_wait(unsigned long long* bar, unsigned parity, unsigned* fault) {
