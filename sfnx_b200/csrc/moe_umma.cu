@@ -7,15 +7,23 @@
 // half product q * d, :184-216; Q6_K in 32-column units, which the reference's prompt path does not take, by the same
 // rule: one half product (q - 32) * f16(d sc)), activations f16, products summed in fp32.
 //
-// A CTA takes 128 of an expert's rows and one or two of the expert's jobs (consecutive jobs of one expert are paired, so
-// that their weights are dequantised once).  The rows are the M side of tcgen05.mma (kind::f16, cta_group::1, M 128),
-// the jobs' activation rows the N side (16 to 128), and the 128 x N fp32 result sits in tensor memory.  Eight producer
-// warps turn 64 columns at a time into the A operand (128 rows x 128 bytes, K-major, 128-byte swizzle) in one of three
-// shared-memory stages, next to the jobs' activation rows for those columns (the B operand, same form, by cp.async);
-// raw weight bytes are fetched a step ahead into registers (a Q4_K super-block, four stages' worth, at a time).  A
-// ninth warp waits for a stage to be full, issues its four MMAs (K 16 each) and lets tcgen05.commit hand the stage
-// back.  Two CTAs share an SM (97 KB of shared memory and 128 columns of tensor memory each), so one streams while the
-// other starts or drains.  Every wait is bounded and feeds the device fault word.
+// One persistent CTA a multiprocessor walks tiles of 256 of an expert's rows against one or two of the expert's jobs
+// (consecutive jobs of one expert are paired, so that their weights are dequantised once), the tiles of a pair side by side
+// on neighbouring CTAs.  The rows are the M side of tcgen05.mma (kind::f16, cta_group::1, twice M 128), the jobs'
+// activation rows the N side (16 to 128), and the 256 x N fp32 result sits in one of two halves of tensor memory.
+//   warps 0-15   the producers: 64 columns at a time of the weights into the A operand (rows of 128 bytes, K-major, 128-byte
+//                swizzle) in one of three shared-memory stages.  A tile's result is written out after the next
+//                tile's first stages are full, so the tensor cores and the copies never wait for it.
+//   warp 16      issues a full stage's MMAs (K 16 each) and lets tcgen05.commit hand the stage back
+//   warp 17      asks for the raw weights (TMA tensor loads into a ring of their own)
+//   warps 18-23  the jobs' activation rows (the B operand, same form) by asynchronous copies, two warps a stage
+// Every wait is bounded and feeds the device fault word.
+//
+// What bounds it: the producers' dequantisation and the shared-memory pipe (its stores and the weights' 16-byte loads), not
+// the tensor cores or HBM.  256 rows a tile halve the copies of activation rows (against 128 rows and two CTAs an SM), and
+// running on from tile to tile hides a tile's start and end.  4096 tokens (1010 jobs, 512 experts
+// of 1536 x 3072 and 3072 x 768): gate|up Q4_K 1.18 -> 0.87 ms, down Q6_K 0.95 -> 0.69; Q8_0 1.42 -> 0.91 and 0.92 -> 0.58;
+// 130 tokens, Q4_K/Q6_K: 0.92 -> 0.60 and 0.64 -> 0.53.
 #include <algorithm>
 
 #include "common.cuh"
@@ -25,9 +33,11 @@
 
 namespace fnxk {
 
-constexpr int MU_BM = 128, MU_KC = 64, MU_NS = 3, MU_PROD = 256, MU_THREADS = MU_PROD + 32, MU_PAIR = 2, MU_NMAX = MU_PAIR * FNX_PF_JOB;
+constexpr int MU_BM = 256, MU_KC = 64, MU_NS = 3, MU_PROD = 512, MU_COPY = 6, MU_THREADS = MU_PROD + 64 + 32 * MU_COPY, MU_PAIR = 2, MU_NMAX = MU_PAIR * FNX_PF_JOB;
+constexpr int MU_LIST = 2048;   // jobs whose pairs are listed at a time
 constexpr int MU_ABYTES = MU_BM * 128, MU_BBYTES = MU_NMAX * 128, MU_STAGE = MU_ABYTES + MU_BBYTES;
-constexpr size_t MU_SMEM = (size_t) MU_NS * MU_STAGE + 1024;
+constexpr int MU_RAW = 73728;   // the raw weights' ring
+constexpr size_t MU_SMEM = (size_t) MU_NS * MU_STAGE + MU_RAW + 1024 + MU_LIST * 2;
 
 __device__ __forceinline__ void mu_arrive(unsigned long long* bar) {
     asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(um_s32(bar)) : "memory");
@@ -53,40 +63,58 @@ struct MuArgs {
     unsigned* fault;
 };
 
-// The raw bytes of one thread's share, (row, half) of the 128 x 64 weight tile, for STEPS consecutive tiles: a Q4_K
-// super-block (256 columns) is one 16-byte header and four 32-byte runs of quants, so a thread takes its half of all four
-// runs and the header in five loads; the other types are fetched tile by tile.
-template <int TYPE> struct MuRaw {
-    static constexpr int STEPS = 1;
+// The raw weights of a tile: the plane that holds nearly all of them comes through a ring in shared memory by TMA tensor
+// loads, STEPS steps (64 columns each) of the tile's 256 rows a load: Q4_K whole super-blocks (144 bytes a row, four steps;
+// rows 144 bytes apart are conflict-free as they are), Q8_0 the quants (64 bytes, swizzled), Q6_K the low nibbles (32
+// bytes, swizzled).  What is left (scales, Q6_K's high bits) a thread loads for its own row and half, a step ahead.
+// (Every thread loading its own row's pieces put 16 lines into each request and was the slowest part: 0.7 ms of 1.2 for
+// gate|up of 512 experts of 1536 x 3072 with everything else taken out.)
+// volatile: the loads stay where they are written, a step ahead of their use
+__device__ __forceinline__ uint2 mu_ld8(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned mu_ld2(const void* p) {
+    unsigned short v;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+template <int TYPE> struct MuRaw {   // Q8_0, Q6_K
+    static constexpr int STEPS = 1, WIDTH = TYPE == FNX_Q8_0 ? 64 : 32, SLOTS = 4;
     uint4 q0, q1;   // Q8_0: the 32 quants; Q6_K: q0 = low nibbles, q1.xy = high bits
     unsigned s, d;  // Q8_0: s = scale; Q6_K: s = the two scales, d = d
     __device__ __forceinline__ void fetch(const MuArgs& a, int expert, int row, int half, int step) {
         const int k0 = step * MU_KC;
         if (32 * half >= a.ncols - k0) return;   // a last tile of 32 columns
         if (TYPE == FNX_Q8_0) {
-            const int blkc = k0 / 32 + half;
-            const uint4* q = reinterpret_cast<const uint4*>(a.a + (size_t) expert * a.stride + (size_t) row * a.ncols + (size_t) blkc * 32);
-            q0 = __ldg(q);
-            q1 = __ldg(q + 1);
-            s = __ldg(reinterpret_cast<const uint16_t*>(a.b + (size_t) expert * a.stride_b) + (size_t) row * (a.ncols / 32) + blkc);
+            s = mu_ld2(reinterpret_cast<const uint16_t*>(a.b + (size_t) expert * a.stride_b) + (size_t) row * (a.ncols / 32) + k0 / 32 + half);
         } else {
             const size_t g = (size_t) expert * a.stride + (size_t) row * (a.ncols / 32) + k0 / 32 + half;
-            q0 = __ldg(reinterpret_cast<const uint4*>(a.a) + g);
-            const uint2 h = __ldg(reinterpret_cast<const uint2*>(a.b) + g);
+            const uint2 h = mu_ld8(reinterpret_cast<const uint2*>(a.b) + g);
             q1.x = h.x, q1.y = h.y;
-            s = __ldg(reinterpret_cast<const uint16_t*>(a.c) + g);
-            d = __ldg(reinterpret_cast<const uint16_t*>(a.d) + g);
+            s = mu_ld2(reinterpret_cast<const uint16_t*>(a.c) + g);
+            d = mu_ld2(reinterpret_cast<const uint16_t*>(a.d) + g);
+        }
+    }
+    __device__ __forceinline__ void begin(const unsigned char*, int) {}
+    __device__ __forceinline__ void read(const unsigned char* slot, int row, int half, int) {   // the swizzles of 64 and 32 bytes
+        if (TYPE == FNX_Q8_0) {
+            const uint4* r = reinterpret_cast<const uint4*>(slot + row * 64);
+            const int sw = (row >> 1) & 3;
+            q0 = r[(2 * half) ^ sw], q1 = r[(2 * half + 1) ^ sw];
+        } else {
+            q0 = reinterpret_cast<const uint4*>(slot + row * 32)[half ^ ((row >> 2) & 1)];
         }
     }
 };
 template <> struct MuRaw<FNX_Q4_K> {
-    static constexpr int STEPS = 4;
+    static constexpr int STEPS = 4, WIDTH = 144, SLOTS = 2;
     uint4 hd, q[4];
-    __device__ __forceinline__ void fetch(const MuArgs& a, int expert, int row, int half, int step) {
-        const unsigned char* blk = a.a + (size_t) expert * a.stride + ((size_t) row * (a.ncols / 256) + step) * 144;
-        hd = __ldg(reinterpret_cast<const uint4*>(blk));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) q[j] = __ldg(reinterpret_cast<const uint4*>(blk + 16 + 32 * j + 16 * half));
+    __device__ __forceinline__ void fetch(const MuArgs&, int, int, int, int) {}
+    __device__ __forceinline__ void begin(const unsigned char* slot, int row) { hd = *reinterpret_cast<const uint4*>(slot + row * 144); }
+    __device__ __forceinline__ void read(const unsigned char* slot, int row, int half, int j) {
+        q[j] = *reinterpret_cast<const uint4*>(slot + row * 144 + 16 + 32 * j + 16 * half);
     }
 };
 
@@ -157,152 +185,279 @@ __device__ __forceinline__ void mu_dequant(const MuRaw<FNX_Q6_K>& r, int, unsign
     mu_put(tile, row, 4 * half + 3, hi[4], hi[5], hi[6], hi[7]);
 }
 
+// The first jobs of the pairs among jobs [base, base + cnt), cnt <= MU_LIST, in order; all threads.  An expert's jobs are
+// consecutive and are paired from its first one; `run`: where the run of the job before `base` began.
+__device__ int mu_list_pairs(const FnxBigJob* jobs, int base, int cnt, int& run, uint16_t* list) {
+    __shared__ int wstart[MU_THREADS / 32], wcount[MU_THREADS / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int per = (cnt + MU_THREADS - 1) / MU_THREADS, lo = base + min(cnt, tid * per), hi = base + min(cnt, (tid + 1) * per);
+    int start = -1;   // the last run that begins among this thread's jobs
+    for (int j = lo; j < hi; ++j)
+        if (j == 0 || jobs[j].w != jobs[j - 1].w) start = j;
+    int before = start;   // the last run that begins at or before this thread's jobs
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before = max(before, v);
+    }
+    if (lane == 31) wstart[warp] = before;
+    before = __shfl_up_sync(0xffffffffu, before, 1);
+    if (lane == 0) before = -1;
+    __syncthreads();
+    int last = run;
+    for (int w = 0; w < MU_THREADS / 32; ++w) {
+        if (w < warp) before = max(before, wstart[w]);
+        last = max(last, wstart[w]);
+    }
+    before = max(before, run);
+    auto is_first = [&](int j, int& at) {
+        if (j == 0 || jobs[j].w != jobs[j - 1].w) at = j;
+        return ((j - at) & 1) == 0;
+    };
+    int n = 0, at = before;
+    for (int j = lo; j < hi; ++j) n += is_first(j, at);
+    int pre = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += v;
+    }
+    if (lane == 31) wcount[warp] = pre;
+    __syncthreads();
+    int total = 0;
+    pre -= n;
+    for (int w = 0; w < MU_THREADS / 32; ++w) {
+        if (w < warp) pre += wcount[w];
+        total += wcount[w];
+    }
+    at = before;
+    for (int j = lo; j < hi; ++j)
+        if (is_first(j, at)) list[pre++] = (uint16_t) (j - base);
+    run = last;
+    __syncthreads();
+    return total;
+}
+
 // out[jb.out[j] * nrows + row] = sum_k W_e[row][k] x[jb.y[j] * ncols + k]
 template <int TYPE>
-__global__ void __launch_bounds__(MU_THREADS, 2) k_moe_umma(const MuArgs a) {
-    const int ji = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+__global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, const __grid_constant__ CUtensorMap wmap) {
+    using Raw = MuRaw<TYPE>;
+    const int tid = threadIdx.x, warp = (int) um_uniform(tid >> 5), lane = tid & 31;
     const int njobs = *a.njobs;
-    if (ji >= njobs) return;
-    // Consecutive jobs of one expert share the dequantised weights: the jobs of an expert are taken two at a time, the
-    // first of a pair does both (its rows in columns 0..63 of the result, the partner's from column 64), the second
-    // leaves at once.  A pair is counted from the expert's first job.
-    const int expert = a.jobs[ji].w;
-    int first = ji;
-    while (first > 0 && a.jobs[first - 1].w == expert) --first;
-    if ((ji - first) & 1) return;
-    const bool paired = ji + 1 < njobs && a.jobs[ji + 1].w == expert;
     extern __shared__ __align__(1024) unsigned char mu_smem[];
     // the swizzle is a function of the shared-memory address: operand tiles start on 1024-byte boundaries
     unsigned char* stages = mu_smem + ((1024u - (um_s32(mu_smem) & 1023u)) & 1023u);
-    __shared__ FnxBigJob jb, jb2;
-    __shared__ __align__(8) unsigned long long full[MU_NS], empty[MU_NS], done;
+    unsigned char* raw = stages + (size_t) MU_NS * MU_STAGE;
+    uint16_t* list = reinterpret_cast<uint16_t*>(raw + MU_RAW);
+    static_assert(MU_COPY == 2 * MU_NS, "two copy warps a stage");
+    static_assert(Raw::SLOTS * Raw::WIDTH * MU_BM <= MU_RAW, "the raw ring");
+    __shared__ __align__(8) unsigned long long full[MU_NS], empty[MU_NS], done[2], freed[2], rfull[Raw::SLOTS], rempty[Raw::SLOTS];
     __shared__ unsigned tmem_base;
-    for (int i = tid; i < (int) (sizeof(FnxBigJob) / 4); i += MU_THREADS) {
-        reinterpret_cast<int*>(&jb)[i] = reinterpret_cast<const int*>(a.jobs + ji)[i];
-        reinterpret_cast<int*>(&jb2)[i] = paired ? reinterpret_cast<const int*>(a.jobs + ji + 1)[i] : 0;
-    }
+    __shared__ int ys[MU_COPY][MU_NMAX / 2];   // a copy warp's rows of x, -1: none
     if (tid == 0) {
         for (int s = 0; s < MU_NS; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&full[s])), "r"(MU_PROD));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&full[s])), "r"(MU_PROD / 32 + 64));   // the producers' warps and two copy warps' lanes
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&empty[s])));
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&done)));
+        for (int s = 0; s < Raw::SLOTS; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&rfull[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&rempty[s])), "r"(MU_PROD / 32));
+        }
+        for (int s = 0; s < 2; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&done[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&freed[s])), "r"(MU_PROD / 32));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == MU_PROD / 32) {   // 128 columns of tensor memory: the 128 x (64 + 64) fp32 result
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(um_s32(&tmem_base)), "r"(MU_NMAX));
+    if (warp == MU_PROD / 32) {   // all 512 columns of tensor memory: two results of 2 x 128 rows x (64 + 64)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(um_s32(&tmem_base)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // a last step of 32 columns (an FF slice of 96) fills half a stage: two MMAs instead of four
-    const int n = min(max(jb.n, 0), FNX_PF_JOB), n2 = paired ? min(max(jb2.n, 0), FNX_PF_JOB) : 0;
-    const int ncol = paired ? FNX_PF_JOB + 16 * ((n2 + 15) / 16) : 16 * ((n + 15) / 16);   // N of the MMAs
-    const int nk = (a.ncols + MU_KC - 1) / MU_KC, row0 = blockIdx.x * MU_BM;
+    const int nk = (a.ncols + MU_KC - 1) / MU_KC, ntiles = (a.nrows + MU_BM - 1) / MU_BM;
     const unsigned st_s = um_s32(stages);
     bool alive = true;   // false after a wait ran out
-    if (warp < MU_PROD / 32) {
-        // ---- producers.  Weights: warp w owns rows 16 w .. + 15 of the tile, lanes 0..15 the first 32 columns of a step
-        // and lanes 16..31 the last 32 (the two lanes of a row read neighbouring bytes: a warp's load touches 16 lines, and
-        // a quarter-warp's stores 8 different rows of one 16-byte column: no bank conflicts).  Activations: 16-byte pieces
-        // tid and tid + 256 of 64 rows x 8, copied asynchronously one step ahead straight into the stage.
-        using Raw = MuRaw<TYPE>;
-        const int row = 16 * warp + (lane & 15), half = lane >> 4;
-        const int wrow = min(row0 + row, a.nrows - 1);   // rows past the matrix repeat the last one; never written out
-        const int xc = tid & 7;
-        const uint16_t* xp[MU_NMAX / 32];   // B rows tid / 8 + 32 i: rows 0..63 the job's, 64..127 its partner's
-        unsigned xd[MU_NMAX / 32];
-#pragma unroll
-        for (int i = 0; i < MU_NMAX / 32; ++i) {
-            const int j = (tid >> 3) + 32 * i, jj = j & (FNX_PF_JOB - 1);
-            const bool has = j < FNX_PF_JOB ? jj < n : jj < n2;
-            xp[i] = has ? a.x + (size_t) (j < FNX_PF_JOB ? jb.y[jj] : jb2.y[jj]) * a.ncols + xc * 8 : nullptr;
-            xd[i] = MU_ABYTES + j * 128 + ((xc ^ (j & 7)) << 4);
-        }
-        auto xcopy = [&](int k) {   // the job's rows for step k, once its stage is free
-            if (k < nk) {
-                const int s = k % MU_NS;
-                if (k >= MU_NS && alive) alive = um_wait(&empty[s], (unsigned) ((k / MU_NS - 1) & 1), a.fault);
-                const unsigned tile = st_s + s * MU_STAGE;
-                const bool in = 8 * xc < a.ncols - k * MU_KC;
-#pragma unroll
-                for (int i = 0; i < MU_NMAX / 32; ++i)
-                    if (xp[i] && in) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tile + xd[i]), "l"(xp[i] + k * MU_KC));
-            }
-            asm volatile("cp.async.commit_group;");
+    unsigned g0 = 0, seq = 0, rc = 0;   // steps, tiles and raw loads that this role has behind it
+    const int nsteps = (nk + Raw::STEPS - 1) / Raw::STEPS;
+    int run = 0;
+    for (int base = 0; base < njobs; base += MU_LIST) {
+        const int items = mu_list_pairs(a.jobs, base, min(MU_LIST, njobs - base), run, list) * ntiles;
+        const int first = blockIdx.x, stride = gridDim.x;
+        auto job_of = [&](int it) { return base + list[it / ntiles]; };
+        // a tile's jobs' rows; n2: the partner's, 0 without one
+        auto rows_of = [&](int ji, int& n, int& n2) {
+            n = min(max(a.jobs[ji].n, 0), FNX_PF_JOB);
+            const bool paired = ji + 1 < njobs && a.jobs[ji + 1].w == a.jobs[ji].w;
+            n2 = paired ? min(max(a.jobs[ji + 1].n, 0), FNX_PF_JOB) : 0;
         };
-        auto produce = [&](const Raw& r, int j, int k) {
-            xcopy(k + 1);   // also makes sure that the stage the next step writes is free
-            const unsigned tile = st_s + (k % MU_NS) * MU_STAGE;
-            if (32 * half < a.ncols - k * MU_KC) mu_dequant(r, j, tile, row, half);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");          // this step's activation pieces have landed
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes before the tensor core's reads
-            mu_arrive(&full[k % MU_NS]);
-        };
-        const int nsteps = (nk + Raw::STEPS - 1) / Raw::STEPS;
-        Raw r0, r1;
-        r0.fetch(a, expert, wrow, half, 0);
-        xcopy(0);
+        auto cols_of = [&](int n, int n2) { return n2 ? FNX_PF_JOB + 16 * ((n2 + 15) / 16) : 16 * ((n + 15) / 16); };   // N of the MMAs
+        if (warp < MU_PROD / 32) {
+            // ---- producers: warp w owns rows 16 w .. + 15 of the tile, lanes 0..15 the first 32 columns of a step and lanes
+            // 16..31 the last 32 (the two lanes of a row read neighbouring bytes: a warp's load touches 16 lines, and a
+            // quarter-warp's stores 8 different rows of one 16-byte column: no bank conflicts)
+            const int row = 16 * warp + (lane & 15), half = lane >> 4;
+            auto wrow = [&](int it) { return min(it % ntiles * MU_BM + row, a.nrows - 1); };   // rows past the matrix repeat the last one; never written out
+            // the result of tile number t, item `it`, out of tensor memory: warp w reads lanes 32 (w % 4) .. + 31 (its quarter)
+            // of the rows' lower or upper 128, the first or second half of the columns; 32 lanes write 32 consecutive floats
+            auto write_out = [&](int it, unsigned t) {
+                const unsigned buf = t & 1u;
+                const int ji = job_of(it);
+                int n, n2;
+                rows_of(ji, n, n2);
+                if (alive) alive = um_wait(&done[buf], (t >> 1) & 1u, a.fault);
+                const bool ok = __all_sync(0xffffffffu, alive);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int hi = (warp >> 2) & 1, orow = it % ntiles * MU_BM + 128 * hi + 32 * (warp & 3) + lane;
+                const int cols = cols_of(n, n2) / 2, c0 = (warp >> 3) * cols;
+                if (ok)
+                    for (int c = c0; c < c0 + cols; c += 8) {
+                        unsigned v[8];
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                                     : "r"(tmem_base + ((unsigned) (32 * (warp & 3)) << 16) + buf * 256u + 128u * hi + (unsigned) c));
+                        const bool second = c >= FNX_PF_JOB;
+                        const int jj = c & (FNX_PF_JOB - 1), live = second ? n2 : n;
+                        const int4* op = reinterpret_cast<const int4*>(a.jobs[ji + second].out + jj);
+                        int o[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) o[i] = reinterpret_cast<const int*>(op)[i];
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (jj + i < live && orow < a.nrows) a.out[(size_t) o[i] * a.nrows + orow] = __uint_as_float(v[i]);
+                    }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mu_arrive(&freed[buf]);
+            };
+            Raw cur, nxt;
+            if (first < items) cur.fetch(a, a.jobs[job_of(first)].w, wrow(first), half, 0);
+            int prev = -1;
+            for (int it = first; it < items; it += stride, ++seq, g0 += nk) {
+                const int expert = a.jobs[job_of(it)].w, wr = wrow(it);
+                const bool more = it + stride < items;
+                const int nexpert = more ? a.jobs[job_of(it + stride)].w : 0, nwr = more ? wrow(it + stride) : 0;
 #pragma unroll 1
-        for (int sidx = 0; sidx < nsteps; sidx += 2) {
-            if (sidx + 1 < nsteps) r1.fetch(a, expert, wrow, half, sidx + 1);
+                for (int sidx = 0; sidx < nsteps; ++sidx, ++rc) {
+                    if (sidx + 1 < nsteps) nxt.fetch(a, expert, wr, half, sidx + 1);
+                    else if (more) nxt.fetch(a, nexpert, nwr, half, 0);
+                    const unsigned slot = rc % Raw::SLOTS;
+                    const unsigned char* rs = raw + slot * (Raw::WIDTH * MU_BM);
+                    if (alive) alive = um_wait(&rfull[slot], (rc / Raw::SLOTS) & 1u, a.fault);
+                    cur.begin(rs, row);
 #pragma unroll
-            for (int j = 0; j < Raw::STEPS; ++j)
-                if (sidx * Raw::STEPS + j < nk) produce(r0, j, sidx * Raw::STEPS + j);
-            if (sidx + 1 < nsteps) {
-                if (sidx + 2 < nsteps) r0.fetch(a, expert, wrow, half, sidx + 2);
-#pragma unroll
-                for (int j = 0; j < Raw::STEPS; ++j)
-                    if ((sidx + 1) * Raw::STEPS + j < nk) produce(r1, j, (sidx + 1) * Raw::STEPS + j);
+                    for (int j = 0; j < Raw::STEPS; ++j) {
+                        const int k = sidx * Raw::STEPS + j;
+                        if (k < nk) {
+                            const unsigned g = g0 + k, s = g % MU_NS;
+                            cur.read(rs, row, half, j);
+                            if (g >= MU_NS && alive) alive = um_wait(&empty[s], (g / MU_NS - 1) & 1u, a.fault);
+                            if (32 * half < a.ncols - k * MU_KC) mu_dequant(cur, j, st_s + s * MU_STAGE + (row >> 7) * 16384, row & 127, half);
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes before the tensor core's reads
+                            __syncwarp();
+                            if (lane == 0) mu_arrive(&full[s]);
+                        }
+                    }
+                    if (lane == 0) mu_arrive(&rempty[slot]);   // every lane's reads lie before the last step's warp barrier
+                    cur = nxt;
+                    if (prev >= 0 && ((sidx + 1) * Raw::STEPS >= MU_NS - 1 || sidx + 1 == nsteps)) {
+                        write_out(prev, seq - 1);
+                        prev = -1;
+                    }
+                }
+                prev = it;
             }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else {
-        // ---- the issuing warp: stage k's four MMAs once it is full; the commit frees the stage
-        const unsigned idesc = (1u << 4) | ((unsigned) (ncol >> 3) << 17) | ((128u >> 4) << 24);   // D f32, A and B f16 K-major
+            if (prev >= 0) write_out(prev, seq - 1);
+        } else if (warp == MU_PROD / 32 + 1) {
+            // ---- the raw weights' loads, as far ahead as the ring holds, across the ends of tiles
+            if (lane == 0)
+                for (int it = first; it < items; it += stride) {
+                    const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
+                    for (int c = 0; c < nsteps; ++c, ++rc) {
+                        const unsigned slot = rc % Raw::SLOTS;
+                        if (rc >= Raw::SLOTS && alive) alive = um_wait(&rempty[slot], (rc / Raw::SLOTS - 1) & 1u, a.fault);
+                        um_expect_tx(&rfull[slot], Raw::WIDTH * MU_BM);
+                        um_tma3d(um_s32(raw + slot * (Raw::WIDTH * MU_BM)), &wmap, c * Raw::WIDTH, it % ntiles * MU_BM, expert, &rfull[slot]);
+                    }
+                }
+        } else if (warp > MU_PROD / 32) {
+            // ---- the activation rows, by asynchronous copies, two warps a step in turn: every stage's copies are issued side by side.  Lane i takes
+            // the 16-byte piece i % 8 of rows i / 8 (+ 4 in the second warp), + 8, ... of the stage's 128 (0..63 the job's, 64..127 its partner's)
+            const unsigned mine = (warp - MU_PROD / 32 - 2) >> 1;
+            const int xc = lane & 7, r0 = (lane >> 3) + 4 * ((warp - MU_PROD / 32) & 1);
+            for (int it = first; it < items; it += stride, g0 += nk) {
+                const int ji = job_of(it);
+                int n, n2;
+                rows_of(ji, n, n2);
+                const FnxBigJob &jb = a.jobs[ji], &jb2 = a.jobs[n2 ? ji + 1 : ji];
+                __syncwarp();
+                int* yw = ys[warp - MU_PROD / 32 - 2];   // [i][lane / 8]: row r0 + 8 i
+                for (int q = lane; q < MU_NMAX / 2; q += 32) {   // the rows' indices, for every step of the tile
+                    const int j = (q & 3) + 4 * ((warp - MU_PROD / 32) & 1) + 8 * (q >> 2);
+                    yw[q] = j < FNX_PF_JOB ? (j < n ? jb.y[j] : -1) : (j - FNX_PF_JOB < n2 ? jb2.y[j - FNX_PF_JOB] : -1);
+                }
+                __syncwarp();
 #pragma unroll 1
-        for (int k = 0; k < nk; ++k) {
-            const int s = k % MU_NS;
-            if (alive) alive = um_wait(&full[s], (unsigned) ((k / MU_NS) & 1), a.fault);
-            alive = __all_sync(0xffffffffu, alive);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
-                const unsigned long long da = um_desc(st_s + s * MU_STAGE), db = um_desc(st_s + s * MU_STAGE + MU_ABYTES);
-#pragma unroll
-                for (int ks = 0; ks < MU_KC / 16; ++ks)
-                    if (16 * ks < a.ncols - k * MU_KC) um_mma(tmem_base, da + 2 * ks, db + 2 * ks, idesc, (unsigned) (k | ks));
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&empty[s])) : "memory");
-            }
-            __syncwarp();
-        }
-        if (lane == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&done)) : "memory");
-    }
-    // ---- the result out of tensor memory: warp w reads lanes 32 (w % 4) .. + 31 (its quarter), rows of the tile; warps
-    // 0..3 take the first half of the job's rows, warps 4..7 the second; a warp's 32 lanes write 32 consecutive floats
-    if (warp < MU_PROD / 32) {
-        bool ok = alive && um_wait(&done, 0u, a.fault);
-        ok = __all_sync(0xffffffffu, ok);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = row0 + 32 * (warp & 3) + lane, cols = ncol / 2, c0 = (warp >> 2) * cols;
-        if (ok)
-            for (int c = c0; c < c0 + cols; c += 8) {
-                unsigned v[8];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                             : "r"(tmem_base + ((unsigned) (32 * (warp & 3)) << 16) + (unsigned) c));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int col = c + i, jj = col & (FNX_PF_JOB - 1);
-                    const bool second = paired && col >= FNX_PF_JOB;
-                    if (jj < (second ? n2 : n) && row < a.nrows) a.out[(size_t) (second ? jb2.out[jj] : jb.out[jj]) * a.nrows + row] = __uint_as_float(v[i]);
+                for (int k = (int) ((mine + MU_NS - g0 % MU_NS) % MU_NS); k < nk; k += MU_NS) {
+                    const unsigned g = g0 + k, s = g % MU_NS;
+                    if (g >= MU_NS && alive) alive = um_wait(&empty[s], (g / MU_NS - 1) & 1u, a.fault);
+                    const unsigned tile = st_s + s * MU_STAGE + MU_ABYTES;
+                    const uint16_t* xk = a.x + (size_t) k * MU_KC + 8 * xc;
+                    if (8 * xc < a.ncols - k * MU_KC) {
+#pragma unroll 4
+                        for (int j = r0; j < (n2 ? FNX_PF_JOB + n2 : n); j += 8) {
+                            const int y = yw[(j >> 3) * 4 + (lane >> 3)];
+                            if (y >= 0)
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tile + j * 128 + ((xc ^ (j & 7)) << 4)), "l"(xk + (size_t) y * a.ncols));
+                        }
+                    }
+                    // the lane's arrival, made by the copies' unit when they have landed (the issuing warp fences them)
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(um_s32(&full[s])) : "memory");
                 }
             }
+        } else {
+            // ---- the issuing warp: a stage's MMAs once it is full; the commit frees the stage
+            for (int it = first; it < items; it += stride, ++seq, g0 += nk) {
+                int n, n2;
+                rows_of(job_of(it), n, n2);
+                const unsigned idesc = (1u << 4) | ((unsigned) (cols_of(n, n2) >> 3) << 17) | ((128u >> 4) << 24);   // D f32, A and B f16 K-major
+                const unsigned d = um_uniform(tmem_base) + (seq & 1u) * 256u;
+                const bool upper = it % ntiles * MU_BM + 128 < a.nrows;
+                if (seq >= 2 && alive) alive = um_wait(&freed[seq & 1u], ((seq >> 1) - 1) & 1u, a.fault);
+#pragma unroll 1
+                for (int k = 0; k < nk; ++k) {
+                    const unsigned g = g0 + k, s = g % MU_NS;
+                    if (alive) alive = um_wait(&full[s], (g / MU_NS) & 1u, a.fault);
+                    alive = __all_sync(0xffffffffu, alive);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copied rows before the tensor core's reads
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (um_elect()) {
+                        const unsigned long long da = um_desc(st_s + s * MU_STAGE), db = um_desc(st_s + s * MU_STAGE + MU_ABYTES);
+                        const int steps = min(MU_KC, a.ncols - k * MU_KC) / 16;
+#pragma unroll
+                        for (int ks = 0; ks < MU_KC / 16; ++ks)
+                            if (ks < steps) {
+                                um_mma(d, da + 2 * ks, db + 2 * ks, idesc, (unsigned) (k | ks));
+                                if (upper) um_mma(d + 128, da + 1024 + 2 * ks, db + 2 * ks, idesc, (unsigned) (k | ks));   // 128 rows on: 16 384 bytes
+                            }
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&empty[s])) : "memory");
+                    }
+                    __syncwarp();
+                }
+                if (um_elect())
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&done[seq & 1u])) : "memory");
+                __syncwarp();
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");   // only a wait that ran out leaves copies in flight here
+        __syncthreads();   // the list may be rewritten
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == MU_PROD / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(MU_NMAX));
+    if (warp == MU_PROD / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
 }
 
 // h = silu(gate) * up of the stacked rows, rounded to f16 (reference src/moe_mma.cuh:381-388)
@@ -323,21 +478,36 @@ static int moe_umma(const char* what, const FnxExperts* A, const FnxBigJob* jobs
     FNX_REQUIRE(fault, "%s: no device fault word (no current device?)", what);
     MuArgs a{A->type, A->nrows, A->ncols, (const unsigned char*) A->a, (const unsigned char*) A->b, (const unsigned char*) A->c,
              (const unsigned char*) A->d, A->stride, A->stride_b, jobs, njobs, x, out, fault};
-    const dim3 grid((A->nrows + MU_BM - 1) / MU_BM, njobs_cap);
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return fail("%s: no device", what);
+    const int grid = (int) std::min<long long>(nsm, (long long) ((A->nrows + MU_BM - 1) / MU_BM) * njobs_cap);
+    // the raw weights' plane as bytes (column, row, expert); how many experts there are is the jobs' business
+    CUtensorMap wmap;
+    const UmEncode encode = um_encoder();
+    FNX_REQUIRE(encode, "%s: the driver has no tensor-map encoder", what);
+    const auto map = [&](int row_bytes, size_t expert_bytes, int width, CUtensorMapSwizzle swizzle) {
+        const cuuint64_t dims[3] = {(cuuint64_t) row_bytes, (cuuint64_t) A->nrows, 1u << 20}, strides[2] = {(cuuint64_t) row_bytes, (cuuint64_t) (expert_bytes ? expert_bytes : row_bytes)};
+        const cuuint32_t box[3] = {(cuuint32_t) width, MU_BM, 1}, ones[3] = {1, 1, 1};
+        return encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(A->a), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
 #define MU_LAUNCH(T)                                                            \
     if (smem_optin(k_moe_umma<T>, MU_SMEM, what)) return 1;                     \
-    k_moe_umma<T><<<grid, MU_THREADS, MU_SMEM, st>>>(a);                        \
+    k_moe_umma<T><<<grid, MU_THREADS, MU_SMEM, st>>>(a, wmap);                        \
     return launch_ok(what);
     if (A->type == FNX_Q4_K) {
         FNX_REQUIRE(A->ncols % 256 == 0 && ((uintptr_t) A->a % 16) == 0 && A->stride % 16 == 0, "%s q4_K: %d columns, rows 16-byte aligned", what, A->ncols);
+        FNX_REQUIRE(map(A->ncols / 256 * 144, A->stride, 144, CU_TENSOR_MAP_SWIZZLE_NONE), "%s q4_K: tensor map", what);
         MU_LAUNCH(FNX_Q4_K)
     }
     if (A->type == FNX_Q8_0) {
         FNX_REQUIRE(((uintptr_t) A->a % 16) == 0 && A->stride % 16 == 0 && A->stride_b % 2 == 0, "%s q8_0: planes 16-byte aligned", what);
+        FNX_REQUIRE(map(A->ncols, A->stride, 64, CU_TENSOR_MAP_SWIZZLE_64B), "%s q8_0: tensor map", what);
         MU_LAUNCH(FNX_Q8_0)
     }
     if (A->type == FNX_Q6_K) {
         FNX_REQUIRE(((uintptr_t) A->a % 16) == 0 && ((uintptr_t) A->b % 8) == 0, "%s q6_K: unit planes not aligned", what);
+        FNX_REQUIRE(map(A->ncols / 2, A->stride * 16, 32, CU_TENSOR_MAP_SWIZZLE_32B), "%s q6_K: tensor map", what);
         MU_LAUNCH(FNX_Q6_K)
     }
 #undef MU_LAUNCH

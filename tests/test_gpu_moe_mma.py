@@ -88,7 +88,8 @@ def test_f16_weights_bit_exact_through_one_hot_rows(kind):
 
 
 @pytest.mark.parametrize("kind,n,ffs,nexp,ntok,topk", [("q4k", 512, 256, 8, 150, 4), ("q8_0", 1024, 96, 6, 70, 3), ("q4k", 3072, 768, 4, 150, 2),
-                                                      ("q4k", 256, 64, 5, 1, 2), ("q8_0", 256, 64, 2, 330, 2)])
+                                                      ("q4k", 256, 64, 5, 1, 2), ("q8_0", 256, 64, 2, 330, 2),
+                                                      ("q8_0", 256, 32, 3, 40, 2), ("q4k", 256, 32, 3, 40, 2)])
 def test_gate_up_swiglu_down(kind, n, ffs, nexp, ntok, topk):
     """gate|up -> SwiGLU -> down over jobs of 1 to 64 rows (ragged job sizes, row tiles past the matrix's last row, FF slice
     96; experts with one, two and six jobs: consecutive jobs of an expert are taken in pairs), each step against the
@@ -122,3 +123,28 @@ def test_gate_up_swiglu_down(kind, n, ffs, nexp, ntok, topk):
     part = _run("fnx_moe_down_mma", ex, dn_jobs, h, P)
     ref, mag = O.moe_mma(_weights16(w, "dn"), dn_jobs, len(dn_jobs), h, n, P)
     _close(part, ref, mag, ffs)
+
+
+@pytest.mark.parametrize("njobs,nexp", [(5000, 7), (2049, 1), (2048, 3), (600, 600)])
+def test_many_jobs(njobs, nexp):
+    """More jobs than are listed at a time (2048): runs of one expert's jobs of every parity, some across the lists' ends, one
+    expert for all, an expert a job; a tile's two jobs with one to three rows each."""
+    from oracle import binding as O
+
+    n, rows = 256, 128
+    rng = np.random.default_rng(njobs)
+    w = cases.moe_weights_q8(n=n, nexp=nexp, ffs=rows // 2, seed=41)
+    lens = rng.integers(1, 3 if nexp > 500 else 40, njobs)
+    run = np.arange(njobs) if nexp == njobs else np.repeat(np.arange(njobs), lens)[:njobs]
+    jobs = np.zeros(njobs, O.BIGJOB_DTYPE)
+    P = 0
+    x16 = _f16_bits(rng.standard_normal((97, n)))
+    for j in range(njobs):
+        k = int(rng.integers(1, 4))
+        jobs[j]["w"], jobs[j]["n"] = run[j] % nexp, k
+        jobs[j]["y"][:k], jobs[j]["out"][:k] = rng.integers(0, 97, k), np.arange(P, P + k)
+        P += k
+    ex, keep = _experts(w, "gu")
+    got = _run("fnx_moe_gate_up_mma", ex, jobs, x16, P)
+    ref, mag = O.moe_mma(_weights16(w, "gu"), jobs, njobs, x16, rows, P)
+    _close(got, ref, mag, n)
