@@ -469,6 +469,22 @@ __global__ void __launch_bounds__(256) k_swiglu_h16(const float* __restrict__ gu
     }
 }
 
+// the same for rows of whole 16-byte pieces: eight values a thread, in flight together.  Bound by HBM (10 bytes a value); a
+// value a thread with a 64-bit division each ran at 2.0 TB/s (40 960 rows of 768: 157 us, now 59).
+__global__ void __launch_bounds__(256) k_swiglu_h16_v8(const float4* __restrict__ gu, unsigned f8, unsigned total, uint4* __restrict__ h) {
+    const unsigned e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= total) return;
+    const unsigned r = e / f8, i = e - r * f8;
+    const float4* g = gu + (size_t) r * 4 * f8 + 2 * i;
+    const float4 g0 = __ldcs(g), g1 = __ldcs(g + 1), u0 = __ldcs(g + 2 * f8), u1 = __ldcs(g + 2 * f8 + 1);
+    const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    unsigned o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        o[k] = f2h(fmul(ex_silu(gv[2 * k]), uv[2 * k])) | (unsigned) f2h(fmul(ex_silu(gv[2 * k + 1]), uv[2 * k + 1])) << 16;
+    h[e] = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 static int moe_umma(const char* what, const FnxExperts* A, const FnxBigJob* jobs, const int* njobs, int njobs_cap, const uint16_t* x, float* out,
                     cudaStream_t st) {
     FNX_REQUIRE(A && jobs && njobs && njobs_cap >= 1 && x && out, "%s: no experts, jobs, rows or output", what);
@@ -528,6 +544,11 @@ int fnx_swiglu_h16(const float* gu, int ffs, int P, uint16_t* h16, void* st) {
     FNX_REQUIRE(gu && h16 && ffs >= 1 && P >= 0, "swiglu_h16: %d rows of %d", P, ffs);
     if (!P) return 0;
     const size_t total = (size_t) P * ffs;
+    if (ffs % 8 == 0 && (uintptr_t) gu % 16 == 0 && (uintptr_t) h16 % 16 == 0 && total / 8 < (1ull << 31)) {
+        const unsigned pieces = (unsigned) (total / 8);
+        k_swiglu_h16_v8<<<(pieces + 255) / 256, 256, 0, strm(st)>>>((const float4*) gu, ffs / 8, pieces, (uint4*) h16);
+        return launch_ok("swiglu_h16");
+    }
     k_swiglu_h16<<<(unsigned) std::min<size_t>(4096, (total + 255) / 256), 256, 0, strm(st)>>>(gu, ffs, total, h16);
     return launch_ok("swiglu_h16");
 }
