@@ -25,8 +25,11 @@
 // instead of 17 (+2 for a rollback).
 #include <cooperative_groups.h>
 
+#include <cstring>
+
 #include "common.cuh"
 #include "exact_math.cuh"
+#include "moe_internal.cuh"
 
 namespace fnxk {
 
@@ -300,8 +303,7 @@ __global__ void __cluster_dims__(GR_CL, 1, 1) __launch_bounds__(GR_THREADS, 1) k
 // ---- the state after the first n rows of a logged window: S <- g_t S + k_t (x) delta_t for t < n, every element with the
 // very operations the rows kernel applied to it (fmul then ffma), so the bits are those of the window's own states.  Block
 // (value head, job): 256 threads, thread = a quad of columns and 16 rows of it.
-__global__ void __launch_bounds__(256) k_gdn_replay(const FnxGdnReplay* __restrict__ jobs) {
-    const FnxGdnReplay jb = jobs[blockIdx.y];
+__device__ __forceinline__ void gdn_replay_job(const FnxGdnReplay& jb) {
     const int lv = blockIdx.x, tid = threadIdx.x, cq = tid & 31, rb = tid >> 5;
     if (lv >= jb.nv || jb.n <= 0) return;
     const int kh = jb.vmap[lv] & 255;
@@ -332,6 +334,31 @@ __global__ void __launch_bounds__(256) k_gdn_replay(const FnxGdnReplay* __restri
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) *reinterpret_cast<float4*>(Sh + (size_t) (rb + 8 * i) * HS) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+}
+__global__ void __launch_bounds__(256) k_gdn_replay(const FnxGdnReplay* __restrict__ jobs) {
+    pdl_wait();
+    pdl_go();
+    gdn_replay_job(jobs[blockIdx.y]);
+}
+// the same with the table as the launch's parameters: no upload ahead of it
+struct ReplayTable {
+    FnxGdnReplay job[64];
+};
+__global__ void __launch_bounds__(256) k_gdn_replay_table(const __grid_constant__ ReplayTable table) {
+    pdl_wait();
+    pdl_go();
+    gdn_replay_job(table.job[blockIdx.y]);
+}
+int gdn_replay_host(const FnxGdnReplay* jobs, int n, int nv_max, cudaStream_t st) {
+    constexpr int CAP = sizeof(ReplayTable) / sizeof(FnxGdnReplay);
+    for (int at = 0; at < n; at += CAP) {
+        ReplayTable t;
+        const int k = n - at < CAP ? n - at : CAP;
+        memcpy(t.job, jobs + at, k * sizeof(FnxGdnReplay));
+        launch(0, k_gdn_replay_table, dim3(nv_max, k), 256, 0, st, t);
+        if (launch_ok("gdn_replay")) return 1;
+    }
+    return 0;
 }
 
 static int gdn_launch(const GdnArgs& g, int nseg, cudaStream_t st, const char* what) {

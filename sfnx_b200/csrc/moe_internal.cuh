@@ -16,6 +16,10 @@ int attn_umma_launch(const float* qg, const uint16_t* kc, const uint16_t* vc, Fn
 int q8s_umma_launch(const FnxQ8S* w, const int* rows, float* const* out, const int* out_stride, int nseg, int cols, const void* yq, int T, cudaStream_t st,
                     const char* what);
 
+// util.cu, gdn.cu: fnx_copy_many and fnx_gdn_replay for a table in host memory, passed in the launches' parameters
+int copy_many_host(const FnxCopyJob* jobs, int n, cudaStream_t st);
+int gdn_replay_host(const FnxGdnReplay* jobs, int n, int nv_max, cudaStream_t st);
+
 // where a kernel with bounded on-chip waits reports a wait that ran out (bit 8): the window's error word while a window
 // stage is being enqueued (fault_sink), else the library's own word, which fnx_device_fault() reads and clears
 unsigned* device_fault_word();

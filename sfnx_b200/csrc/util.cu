@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "exact_math.cuh"
+#include "moe_internal.cuh"
 
 namespace fnxk {
 
@@ -113,14 +114,36 @@ __global__ void __launch_bounds__(1024) k_rms_norm_rows(float* __restrict__ x, c
 }
 
 // ---------------------------------------------------------------- batched copies (reference src/kernels.cu:1473-1485)
-__global__ void __launch_bounds__(256) k_copy_many(const FnxCopyJob* __restrict__ jobs) {
-    pdl_wait();
-    pdl_go();
-    const FnxCopyJob j = jobs[blockIdx.y];
+__device__ __forceinline__ void copy_job(const FnxCopyJob& j) {
     float4* d = reinterpret_cast<float4*>(j.dst);
     const float4* s = reinterpret_cast<const float4*>(j.src);
     const size_t n = j.bytes / 16, step = (size_t) gridDim.x * blockDim.x;
     for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) d[i] = s[i];
+}
+__global__ void __launch_bounds__(256) k_copy_many(const FnxCopyJob* __restrict__ jobs) {
+    pdl_wait();
+    pdl_go();
+    copy_job(jobs[blockIdx.y]);
+}
+// the same with the table as the launch's parameters: no upload ahead of it
+struct CopyTable {
+    FnxCopyJob job[96];
+};
+__global__ void __launch_bounds__(256) k_copy_table(const __grid_constant__ CopyTable table) {
+    pdl_wait();
+    pdl_go();
+    copy_job(table.job[blockIdx.y]);
+}
+int copy_many_host(const FnxCopyJob* jobs, int n, cudaStream_t st) {
+    constexpr int CAP = sizeof(CopyTable) / sizeof(FnxCopyJob);
+    for (int at = 0; at < n; at += CAP) {
+        CopyTable t;
+        const int k = n - at < CAP ? n - at : CAP;
+        memcpy(t.job, jobs + at, k * sizeof(FnxCopyJob));
+        launch(0, k_copy_table, dim3(74, k), 256, 0, st, t);
+        if (launch_ok("copy_many")) return 1;
+    }
+    return 0;
 }
 
 // ---------------------------------------------------------------- L2 prefetch (reference src/kernels.cu:2173-2193)

@@ -86,7 +86,7 @@ struct Traced {
 // the workspace's buffers, as offsets from its base
 struct Ws {
     size_t x, bo, xn, xq, qkvz, ab, yq, qg, k, v, att, partials, att_scratch, rlogits, topi, topw, jobs_gu, jobs_dn, njobs, rscratch, gu,
-        hq, part, sh_gu, shq, sh, logits, keys, best_v, best_i, err, ctl, gdn_scratch, copy_jobs, replay_jobs, hc_R, hc_inj, hc_scratch, dr_en, dr_e2, dr_h2, dr_q, qsa_y, qsa_q, qsa_scores, qsa_cells, qsa_ncells, total;
+        hq, part, sh_gu, shq, sh, logits, keys, best_v, best_i, err, ctl, gdn_scratch, copy_jobs, hc_R, hc_inj, hc_scratch, dr_en, dr_e2, dr_h2, dr_q, qsa_y, qsa_q, qsa_scores, qsa_cells, qsa_ncells, total;
 };
 
 static Ws carve(const FnxStackCfg& c) {
@@ -134,7 +134,6 @@ static Ws carve(const FnxStackCfg& c) {
     w.ctl = take(16);
     w.gdn_scratch = take(fnx_gdn_scratch_floats(c.nv) * 4);
     w.copy_jobs = take((size_t) c.nlayers * 2 * FNX_MAXT * sizeof(FnxCopyJob));   // up to a lane a row
-    w.replay_jobs = take((size_t) c.nlayers * sizeof(FnxGdnReplay));
     const size_t hcn = c.hc > 1 ? (size_t) c.hc : 0;   // hyper-connections: the residual streams, the two halves' inject values, the read's scratch
     w.hc_R = take(T * hcn * n * 4);
     w.hc_inj = take(2 * T * (hcn ? hcn : 1) * 4);
@@ -515,7 +514,6 @@ int fnx_window_commit_lanes(const FnxStackCfg* cfg, const FnxLayer* layers, void
     TRY(check_cfg(cfg));
     FNX_REQUIRE(lanes && n && tags && lanes->S_host && lanes->hist_host, "commit: no lanes");
     const FnxStackCfg& c = *cfg;
-    const Ws w = carve(c);
     FnxCopyJob* hj = (FnxCopyJob*) host_jobs;
     FNX_REQUIRE(hj, "commit: no host job table");
     const size_t ch = (size_t) (2 * c.nk + c.nv) * FNX_HS, state = (size_t) c.nv * FNX_HS * FNX_HS;
@@ -532,17 +530,13 @@ int fnx_window_commit_lanes(const FnxStackCfg* cfg, const FnxLayer* layers, void
         }
     }
     if (!nj) return 0;
-    FnxCopyJob* dj = (FnxCopyJob*) ((char*) ws + w.copy_jobs);
-    if (cudaMemcpyAsync(dj, hj, (size_t) nj * sizeof(FnxCopyJob), cudaMemcpyHostToDevice, strm(st)) != cudaSuccess)
-        return fail("commit: job table upload: %s", cudaGetErrorString(cudaGetLastError()));
-    return fnx_copy_many(dj, nj, st);
+    return copy_many_host(hj, nj, strm(st));
 }
 
 int fnx_window_commit(const FnxStackCfg* cfg, const FnxLayer* layers, void* ws, int T, int n, int tag, void* host_jobs, void* st) {
     TRY(check_cfg(cfg));
     FNX_REQUIRE(T >= 1 && T <= FNX_MAXT && n >= 1 && n <= T, "commit: %d of %d rows", n, T);
     const FnxStackCfg& c = *cfg;
-    const Ws w = carve(c);
     FNX_REQUIRE(host_jobs, "commit: no host job table");
     // the host table: nlayers * 2 copy jobs, then nlayers replay jobs
     FnxCopyJob* hj = (FnxCopyJob*) host_jobs;
@@ -556,19 +550,9 @@ int fnx_window_commit(const FnxStackCfg* cfg, const FnxLayer* layers, void* ws, 
         else if (n < T) hj[nj++] = FnxCopyJob{layers[l].S, layers[l].snap + (size_t) (n - 1) * state, state * 4};
         if (n < T) hj[nj++] = FnxCopyJob{layers[l].hist + (size_t) written * 3 * ch, layers[l].hsnap + (size_t) (n - 1) * 3 * ch, 3 * ch * 4};
     }
-    if (nj) {
-        FnxCopyJob* dj = (FnxCopyJob*) ((char*) ws + w.copy_jobs);
-        if (cudaMemcpyAsync(dj, hj, (size_t) nj * sizeof(FnxCopyJob), cudaMemcpyHostToDevice, strm(st)) != cudaSuccess)
-            return fail("commit: job table upload: %s", cudaGetErrorString(cudaGetLastError()));
-        TRY(fnx_copy_many(dj, nj, st));
-    }
-    if (nr) {
-        FnxGdnReplay* dr = (FnxGdnReplay*) ((char*) ws + w.replay_jobs);
-        if (cudaMemcpyAsync(dr, hr, (size_t) nr * sizeof(FnxGdnReplay), cudaMemcpyHostToDevice, strm(st)) != cudaSuccess)
-            return fail("commit: replay table upload: %s", cudaGetErrorString(cudaGetLastError()));
-        TRY(fnx_gdn_replay(dr, nr, c.nv, st));
-    }
-    return 0;
+    // the tables go with the launches: an upload each was a copy and a gap between two windows
+    if (nj) TRY(copy_many_host(hj, nj, strm(st)));
+    return nr ? gdn_replay_host(hr, nr, c.nv, strm(st)) : 0;
 }
 
 // the side stream and the two events the forks use (null stream: everything on the window's stream)

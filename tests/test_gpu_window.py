@@ -427,3 +427,41 @@ def test_window_of_several_sequences_equals_each_alone(monkeypatch, qsa_top):
     for i in range(nseg):
         for l in gdn:
             assert torch.equal(lanes.S[l][i], want[i][3][l][0]) and torch.equal(lanes.hist[l][i], want[i][3][l][1]), ("cut", i, l)
+
+
+@pytest.mark.parametrize("nlayers,n,log", [(1, 3, False), (48, 1, False), (49, 3, False), (64, 2, True), (65, 4, True), (130, 4, True)])
+def test_commit_tables_of_any_length(nlayers, n, log):
+    """A commit's copies and replays go with the launches in tables of 96 and 64: stacks at and past those lengths, against
+    the same jobs one at a time from device tables."""
+    import ctypes as C
+
+    import torch
+
+    from sfnx_b200 import lib as L
+
+    T, tag, ch = 4, 1, 3 * 128
+    g = torch.Generator("cuda").manual_seed(nlayers)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")   # noqa: E731
+    cfg = L.StackCfg(n=512, nexp=32, topk=2, ff=32, nk=1, nv=1, nq=1, nkv=1, hd=256, nrot=64, vocab_rows=32, nlayers=nlayers, ncard=1, eps=1e-6)
+    layers, S = (L.Layer * nlayers)(), rand(nlayers, 1, 128, 128)
+    hist, hsnap, snap = rand(nlayers, 2, 3, ch), rand(nlayers, 16, 3, ch), rand(nlayers, T, 1, 128, 128)
+    logs, vmap = rand(nlayers, L.load().fnx_gdn_log_floats(1, 1)) * 0.1, torch.zeros(1, dtype=torch.int32, device="cuda")
+    for l in range(nlayers):
+        layers[l].kind, layers[l].vmap = 0, vmap.data_ptr()
+        layers[l].S, layers[l].hist, layers[l].hsnap, layers[l].snap = S[l].data_ptr(), hist[l].data_ptr(), hsnap[l].data_ptr(), snap[l].data_ptr()
+        layers[l].gdn_log = logs[l].data_ptr() if log else None
+    want_S, want_hist = S.clone(), hist.clone()
+    want_hist[:, (tag & 1) ^ 1] = hsnap[:, n - 1] if n < T else want_hist[:, (tag & 1) ^ 1]
+    if not log:
+        want_S = snap[:, n - 1].clone() if n < T else want_S
+    else:
+        for l in range(nlayers):
+            job = L.GdnReplay(want_S[l].data_ptr(), logs[l].data_ptr(), vmap.data_ptr(), 1, 1, 0, n)
+            table = torch.frombuffer(bytearray(bytes(job)), dtype=torch.uint8).cuda()
+            L.call("fnx_gdn_replay", table.data_ptr(), 1, 1, L.stream())
+            torch.cuda.synchronize()
+    ws = torch.zeros(L.load().fnx_window_workspace_bytes(C.byref(cfg)), dtype=torch.uint8, device="cuda")
+    host = torch.zeros(nlayers * (2 * C.sizeof(L.CopyJob) + C.sizeof(L.GdnReplay)), dtype=torch.uint8).pin_memory()
+    L.call("fnx_window_commit", C.byref(cfg), layers, ws.data_ptr(), T, n, tag, host.data_ptr(), L.stream())
+    torch.cuda.synchronize()
+    assert torch.equal(hist, want_hist) and torch.equal(S, want_S)
