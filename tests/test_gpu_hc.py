@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,n,hc,lr,fold,inject", [(16, 3072, 4, 320, True, True), (16, 2560, 4, 320, True, True), (3, 1024, 2, 64, False, False),
-                                                   (1, 512, 4, 32, True, False), (7, 1536, 3, 96, False, True)])
+                                                   (1, 512, 4, 32, True, False), (7, 1536, 3, 96, False, True),
+                                                   # rows past one batch of eight, slices past eight, streams past four
+                                                   (9, 4608, 5, 64, True, True), (8, 512, 8, 32, True, True)])
 def test_hc_read(T, n, hc, lr, fold, inject):
     import oracle.binding as O
     from sfnx_b200 import lib as L

@@ -127,3 +127,13 @@ def test_mmvq_is_the_job_matvec():
     assert L.load().fnx_mmvq(C.byref(ex), dj.data_ptr(), dn.data_ptr(), P, dxq.data_ptr(), out.data_ptr(), 300, L.stream()) != 0
     e6, keep6 = G.experts_q6p(w["dn_planes"], 512, 128)
     assert L.load().fnx_mmvq(C.byref(e6), dj.data_ptr(), dn.data_ptr(), P, dxq.data_ptr(), out.data_ptr(), 512, L.stream()) != 0
+
+
+@pytest.mark.parametrize("T,topk,nexp", [(1, 1, 32), (2, 10, 64), (2, 16, 32), (3, 4, 96), (5, 16, 512), (9, 3, 32), (16, 1, 64)])
+def test_rows_taken_together_and_picks(T, topk, nexp):
+    """The router at one, two and more rows, first and largest numbers of picks, an expert a lane and sixteen, with ties, and
+    the experts' kernels at the job counts that follow."""
+    w = cases.moe_weights(n=1024, nexp=nexp, ffs=96 if T == 3 else 128, seed=T + topk)
+    w["router"][7] = w["router"][3]   # tied logits: the lower index first
+    x = np.random.default_rng(T).standard_normal((T, 1024)).astype(np.float32)
+    _check(w, x, topk=topk)

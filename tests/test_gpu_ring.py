@@ -268,3 +268,28 @@ def test_window_exchange_gives_up_when_a_peer_never_sends():
     y.fill_(3.0)
     G.sync()
     assert float(G.host(y)[0]) == 3.0
+
+
+@pytest.mark.parametrize("topk,T,width", [(1, 1, 512), (3, 2, 4096), (10, 16, 3072), (11, 3, 96), (16, 5, 2560), (33, 2, 1056)])
+def test_boundary_rows_any_number_of_experts(topk, T, width):
+    """The experts' rows of a column are asked for ten at a time: numbers of experts below, at and past one and several tens,
+    widths with idle columns, against fnx_moe_combine -> fnx_rms_norm_rows, bit for bit."""
+    import torch
+
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    rng = np.random.default_rng(topk * width + T)
+    f32 = lambda *s: G.dev(rng.standard_normal(s).astype(np.float32))   # noqa: E731
+    nexp = 64
+    x1, part, topw, sh, logits, wn = f32(T, width), f32(T * topk, width), f32(T, topk), f32(T, width), f32(T, nexp + 1), f32(width)
+    x2, bo, st = x1.clone(), G.zeros((T, width)), L.stream()
+    y1, y2 = G.zeros((T, width)), G.zeros((T, width))
+    q1, q2 = (torch.zeros(T * (width // 32) * 36, dtype=torch.uint8, device=G.DEV) for _ in range(2))
+    err = torch.zeros(1, dtype=torch.int32, device=G.DEV)
+    L.call("fnx_moe_combine", part.data_ptr(), topw.data_ptr(), sh.data_ptr(), logits.data_ptr(), nexp, bo.data_ptr(), T, width, topk, st)
+    L.call("fnx_rms_norm_rows", x1.data_ptr(), bo.data_ptr(), wn.data_ptr(), y1.data_ptr(), q1.data_ptr(), T, width, 1e-6, st)
+    rows = L.MoeRows(part.data_ptr(), topw.data_ptr(), sh.data_ptr(), logits.data_ptr(), nexp, topk)
+    L.call("fnx_boundary_rows", x2.data_ptr(), None, C.byref(rows), None, wn.data_ptr(), y2.data_ptr(), q2.data_ptr(), T, width, 1e-6, err.data_ptr(), st)
+    G.sync()
+    assert torch.equal(x1.view(torch.int32), x2.view(torch.int32)) and torch.equal(y1.view(torch.int32), y2.view(torch.int32)) and torch.equal(q1, q2)
