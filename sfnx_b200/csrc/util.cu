@@ -85,34 +85,17 @@ __global__ void __launch_bounds__(1024) k_rms_norm_rows(float* __restrict__ x, c
                                                         uint8_t* __restrict__ q, int n, float eps) {
     __shared__ float sh[32];
     float* xr = x + (size_t) blockIdx.x * n;
-    const float* ar = add ? add + (size_t) blockIdx.x * n : nullptr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // A chain of latencies: a thread's first RN columns (rows of up to 12 288 whole: four residual streams of 3072) are asked
-    // for together, their weights before the kernel ahead has finished, and stay in registers for the second half
-    // (a row of 12 288: 8.5 us on the critical path when each was waited for, now 6.8).
-    constexpr int RN = 12;
-    float v[RN], wv[RN], av[RN];
-#pragma unroll
-    for (int k = 0; k < RN; ++k) wv[k] = tid + 1024 * k < n ? __ldg(w + tid + 1024 * k) : 0.f;
     pdl_wait();
     pdl_go();
-#pragma unroll
-    for (int k = 0; k < RN; ++k) {
-        const bool live = tid + 1024 * k < n;
-        v[k] = live ? xr[tid + 1024 * k] : 0.f;
-        av[k] = live && ar ? ar[tid + 1024 * k] : 0.f;
-    }
     float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < RN; ++k) {
-        if (tid + 1024 * k >= n) break;
-        if (ar) xr[tid + 1024 * k] = v[k] = fadd(v[k], av[k]);
-        s = ffma(v[k], v[k], s);
-    }
-    for (int i = tid + 1024 * RN; i < n; i += 1024) {
-        float u = xr[i];
-        if (ar) xr[i] = u = fadd(u, ar[i]);
-        s = ffma(u, u, s);
+    for (int i = tid; i < n; i += 1024) {
+        float v = xr[i];
+        if (add) {
+            v = fadd(v, add[(size_t) blockIdx.x * n + i]);
+            xr[i] = v;
+        }
+        s = ffma(v, v, s);
     }
     s = wsum(s);
     if (lane == 0) sh[warp] = s;
@@ -121,16 +104,13 @@ __global__ void __launch_bounds__(1024) k_rms_norm_rows(float* __restrict__ x, c
 #pragma unroll
     for (int i = 0; i < 32; ++i) tot = fadd(tot, sh[i]);
     const float r = ex_rsqrt(fadd(fdiv(tot, (float) n), eps));
-    auto put = [&](int i, float u) {   // n % 32 == 0: a warp's columns are one q8_1 block
-        if (y) y[(size_t) blockIdx.x * n + i] = u;
-        if (q) q8_1_store(u, q + ((size_t) blockIdx.x * (n / 32) + (i >> 5)) * 36, lane);
-    };
-#pragma unroll
-    for (int k = 0; k < RN; ++k) {
-        if (tid + 1024 * k >= n) break;
-        put(tid + 1024 * k, fmul(fmul(v[k], r), wv[k]));
+    for (int i0 = 0; i0 < n; i0 += 1024) {   // n % 32 == 0: a warp's columns are one q8_1 block
+        const int i = i0 + tid;
+        const bool live = i < n;
+        const float v = live ? fmul(fmul(xr[i], r), w[i]) : 0.f;
+        if (live && y) y[(size_t) blockIdx.x * n + i] = v;
+        if (q && (i0 + warp * 32) < n) q8_1_store(v, q + ((size_t) blockIdx.x * (n / 32) + (i >> 5)) * 36, lane);
     }
-    for (int i = tid + 1024 * RN; i < n; i += 1024) put(i, fmul(fmul(xr[i], r), w[i]));
 }
 
 // ---------------------------------------------------------------- batched copies (reference src/kernels.cu:1473-1485)
