@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
             if (prev >= 0) write_out(prev, seq - 1);
         } else if (warp == MU_PROD / 32 + 1) {
             // ---- the raw weights' loads, as far ahead as the ring holds, across the ends of tiles
-            if (lane == 0)
+            if (lane == 0) {
                 for (int it = first; it < items; it += stride) {
                     const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
                     for (int c = 0; c < nsteps; ++c, ++rc) {
@@ -383,6 +383,9 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
                         um_tma3d(um_s32(raw + slot * (Raw::WIDTH * MU_BM)), &wmap, c * Raw::WIDTH, it % ntiles * MU_BM, expert, &rfull[slot]);
                     }
                 }
+                // no load is in flight when the block ends, also after a wait that ran out
+                for (unsigned k = rc < Raw::SLOTS ? 0 : rc - Raw::SLOTS; k < rc; ++k) um_wait(&rfull[k % Raw::SLOTS], (k / Raw::SLOTS) & 1u, a.fault);
+            }
         } else if (warp > MU_PROD / 32) {
             // ---- the activation rows, by asynchronous copies, two warps a step in turn: every stage's copies are issued side by side.  Lane i takes
             // the 16-byte piece i % 8 of rows i / 8 (+ 4 in the second warp), + 8, ... of the stage's 128 (0..63 the job's, 64..127 its partner's)
