@@ -180,7 +180,8 @@ int fnx_moe_down_noalloc(const FnxExperts* A, const FnxJob* jobs, const int* njo
  * out[jobs[j].out[s]][r] = sum_k f16(W_e[r][k]) * x[jobs[j].y[s]][k] for every job j < *njobs (device) and row s of it; every
  * weight dequantised to f16 with one rounding (Q4_K: q * f16(d sc) - f16(dmin m) as one half fma; Q8_0: q * d; Q6_K in
  * 32-column units: (q - 32) * f16(d sc)), x rows of A->ncols f16 values, fp32 sums on tcgen05 tensor cores (the order
- * of a sum's terms is the hardware's).  A->ncols in units of 32.  njobs_cap: the most jobs there can be (grid rows). */
+ * of a sum's terms is the hardware's).  A->ncols in units of 32.  njobs_cap: the jobs the table holds; a count
+ * above it is taken as njobs_cap. */
 int fnx_moe_gate_up_mma(const FnxExperts* A, const FnxBigJob* jobs, const int* njobs, int njobs_cap, const uint16_t* xh, float* gu,
                         void* st);
 /* h16[p][i] = f16(silu(gu[p][i]) * gu[p][ffs + i]) for P rows of [gate | up] */

@@ -58,6 +58,7 @@ struct MuArgs {
     size_t stride, stride_b;
     const FnxBigJob* jobs;
     const int* njobs;
+    int njobs_cap;   // jobs past it are the caller's other memory, whatever the count on the device says
     const uint16_t* x;
     float* out;
     unsigned* fault;
@@ -243,7 +244,7 @@ template <int TYPE>
 __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, const __grid_constant__ CUtensorMap wmap) {
     using Raw = MuRaw<TYPE>;
     const int tid = threadIdx.x, warp = (int) um_uniform(tid >> 5), lane = tid & 31;
-    const int njobs = *a.njobs;
+    const int njobs = min(*a.njobs, a.njobs_cap);
     extern __shared__ __align__(1024) unsigned char mu_smem[];
     // the swizzle is a function of the shared-memory address: operand tiles start on 1024-byte boundaries
     unsigned char* stages = mu_smem + ((1024u - (um_s32(mu_smem) & 1023u)) & 1023u);
@@ -496,7 +497,7 @@ static int moe_umma(const char* what, const FnxExperts* A, const FnxBigJob* jobs
     unsigned* fault = device_fault_word();
     FNX_REQUIRE(fault, "%s: no device fault word (no current device?)", what);
     MuArgs a{A->type, A->nrows, A->ncols, (const unsigned char*) A->a, (const unsigned char*) A->b, (const unsigned char*) A->c,
-             (const unsigned char*) A->d, A->stride, A->stride_b, jobs, njobs, x, out, fault};
+             (const unsigned char*) A->d, A->stride, A->stride_b, jobs, njobs, njobs_cap, x, out, fault};
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return fail("%s: no device", what);
     const int grid = (int) std::min<long long>(nsm, (long long) ((A->nrows + MU_BM - 1) / MU_BM) * njobs_cap);

@@ -148,3 +148,31 @@ def test_many_jobs(njobs, nexp):
     got = _run("fnx_moe_gate_up_mma", ex, jobs, x16, P)
     ref, mag = O.moe_mma(_weights16(w, "gu"), jobs, njobs, x16, rows, P)
     _close(got, ref, mag, n)
+
+
+@pytest.mark.parametrize("cap,count", [(1, 6), (4, 6), (5, 2048), (2047, 5000), (2049, 5000)])
+def test_no_job_past_the_capacity(cap, count):
+    """A count on the device above the caller's njobs_cap: the jobs up to it are done, those past it (valid ones here, of the
+    same expert as the last) are neither done nor taken as a partner."""
+    import torch
+
+    from oracle import binding as O
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    n, rows = 256, 128
+    w = cases.moe_weights_q8(n=n, nexp=3, ffs=rows // 2, seed=42)
+    jobs = np.zeros(count, O.BIGJOB_DTYPE)
+    jobs["w"], jobs["n"] = np.arange(count) // 3 % 3, 1   # runs of three jobs an expert
+    jobs["y"][:, 0], jobs["out"][:, 0] = np.arange(count) % 97, np.arange(count)
+    x16 = _f16_bits(np.random.default_rng(43).standard_normal((97, n)))
+    ex, keep = _experts(w, "gu")
+    dj, nj, dx = G.dev(jobs.view(np.uint8).reshape(-1)), G.dev(np.array([count, 0], np.int32)), G.dev(x16)
+    out = torch.full((count, rows), float("nan"), device="cuda")
+    L.call("fnx_moe_gate_up_mma", C.byref(ex), dj.data_ptr(), nj.data_ptr(), cap, dx.data_ptr(), out.data_ptr(), L.stream())
+    G.sync()
+    assert L.load().fnx_device_fault() == 0
+    got = G.host(out)
+    ref, mag = O.moe_mma(_weights16(w, "gu"), jobs[:cap], cap, x16, rows, count)
+    _close(got[:cap], ref[:cap], mag[:cap], n)
+    assert np.isnan(got[cap:]).all()
