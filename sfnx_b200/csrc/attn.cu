@@ -465,14 +465,18 @@ __global__ void __launch_bounds__(AxShape<PT>::THREADS, AxShape<PT>::BLOCKS) k_a
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // ---- this run's partial of every pair
+    // ---- this run's partial of every pair, in 8-byte pieces where the caller's scratch allows them
+    const bool pieces = reinterpret_cast<uintptr_t>(acc_out) % 8 == 0;
 #pragma unroll
     for (int i = 0; i < VP; ++i)
         if (vg + i < npt) {
             const int p = pb + vg + i, t = rows_s[p / qpk], h = kvl * qpk + p % qpk;
+            float* o = acc_out + (((size_t) t * nq + h) * ATT_SPLITS + s) * HD + vd;
 #pragma unroll
-            for (int k = 0; k < VD; k += 2)
-                *reinterpret_cast<float2*>(acc_out + (((size_t) t * nq + h) * ATT_SPLITS + s) * HD + vd + k) = make_float2(acc[i][k], acc[i][k + 1]);
+            for (int k = 0; k < VD; k += 2) {
+                if (pieces) *reinterpret_cast<float2*>(o + k) = make_float2(acc[i][k], acc[i][k + 1]);
+                else o[k] = acc[i][k], o[k + 1] = acc[i][k + 1];
+            }
         }
 #pragma unroll
     for (int i = 0; i < PPW; ++i) {

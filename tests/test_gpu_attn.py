@@ -8,8 +8,8 @@ from tests import cases
 pytestmark = pytest.mark.gpu
 
 
-def _run(c, entry="fnx_attn_partial_exact", known_rows=False):
-    """known_rows: the cache is handed over with its row count (FnxKvPages.cap), which lets the tensor-core scan fetch K/V
+def _run(c, entry="fnx_attn_partial_exact", known_rows=False, shift=0):
+    """shift: floats that the scratch begins past a 256-byte boundary.  known_rows: the cache is handed over with its row count (FnxKvPages.cap), which lets the tensor-core scan fetch K/V
     by tensor loads; 70 rows of NaNs are put after the case's rows, inside the count, to stand for stale memory."""
     import torch
 
@@ -34,7 +34,7 @@ def _run(c, entry="fnx_attn_partial_exact", known_rows=False):
             g = L.KvPages(None, 0, 0, c["q8_rows"], 1)
         L.call("fnx_attn_prep_append", qg.data_ptr(), k.data_ptr(), v.data_ptr(), qn.data_ptr(), kn.data_ptr(), kc.data_ptr(),
                vc.data_ptr(), g, card, ncard, T, pos0.data_ptr(), c["eps"], L.Rope(c["rope_base"], 64), nq, nkv, hd, st)
-        scratch = G.zeros(L.load().fnx_attn_scratch_floats(nq, hd, T))
+        scratch = G.zeros(shift + L.load().fnx_attn_scratch_floats(nq, hd, T))[shift:]
         L.call(entry, qg.data_ptr(), kc.data_ptr(), vc.data_ptr(), g, parts[card].data_ptr(), card, ncard, T,
                pos0.data_ptr(), nq, nkv, hd, scratch.data_ptr(), st)
         res["kc"].append(G.host(kc, np.uint16)[:c["kc"][card].shape[0]])
@@ -90,6 +90,17 @@ def test_attention_exact_rows_in_groups_and_slices(T, ctx, hd, q8):
         c = cases.attn_case_q8(c)
     ref, got = cases.attn_oracle(c), _run(c, "fnx_attn_partial_exact")
     assert np.array_equal(got["part"][0].view(np.uint32), ref["part"][0].view(np.uint32))
+
+
+@pytest.mark.parametrize("q8", [False, True])
+@pytest.mark.parametrize("T,ctx,hd,shift", [(16, 300, 256, 1), (1, 300, 256, 1), (5, 100, 128, 3), (2, 100, 128, 2)])
+def test_attention_exact_scratch_at_any_float(T, ctx, hd, shift, q8):
+    """The scratch is an array of floats: one that begins between two 8-byte boundaries gives the same bits."""
+    c = cases.attn_case(T=T, ctx=ctx, nq=12 if hd == 128 else 24, nkv=2 if hd == 128 else 4, hd=hd, seed=60 + T)
+    if q8:
+        c = cases.attn_case_q8(c)
+    got, moved = _run(c), _run(c, shift=shift)
+    assert np.array_equal(got["part"].view(np.uint32), moved["part"].view(np.uint32))
 
 
 @pytest.mark.parametrize("T,ctx,ncard,hd", [(16, 3000, 1, 256), (16, 70, 1, 256), (7, 1500, 2, 256), (5, 515, 4, 128), (1, 0, 1, 256),
