@@ -44,6 +44,8 @@ inline void launch(int kind, void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// brings a line into L2, for what may be written until pdl_wait() returns and so must not be read before it
+__device__ __forceinline__ void l2_ask(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 #endif
 
 #define FNX_REQUIRE(cond, ...) \

@@ -126,10 +126,11 @@ __global__ void __launch_bounds__(HC_DT) k_hc_down(const HcArgs a) {
             wr[4 * q] = v.x, wr[4 * q + 1] = v.y, wr[4 * q + 2] = v.z, wr[4 * q + 3] = v.w;
         }
     }
-    const float wn = t < HC_SL ? __ldg(a.w_norm + col0 + t) : 0.f;
     __shared__ float gate[FNX_MAXT];
+    if (lane == 0 && t < HC_SL) l2_ask(a.w_norm + col0 + t);   // the kernel ahead may still be writing the norm's weights
     pdl_wait();
     pdl_go();
+    const float wn = t < HC_SL ? a.w_norm[col0 + t] : 0.f;
     if (a.bo && t >= HC_SL && t - HC_SL < T) gate[t - HC_SL] = hc_gate(a, t - HC_SL, c);
     // Rows eight at a time: their loads go out together, then their warp sums and maxima interleave (a row at a time, each
     // step of this chain is waited for T times).  Warp w < 16 holds the slice's 32-value block w of every row.

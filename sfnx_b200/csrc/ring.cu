@@ -175,12 +175,15 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_CT) k_boundar
     const int t = blockIdx.x / BD_CL, cr = blockIdx.x % BD_CL, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int vt = cr * BD_CT + tid, n = a.n, nr = a.ring.nrank, me = a.ring.rank;
     float* xr = a.x + (size_t) t * n;
-    float wv[BD_MAXC];   // the norm's weights do not depend on the kernel ahead
 #pragma unroll
-    for (int k = 0; k < BD_MAXC; ++k) wv[k] = __ldg(a.w + min(vt + BD_THREADS * k, n - 1));
+    for (int k = 0; k < BD_MAXC; ++k)   // the norm's weights on their way; the kernel ahead may still be writing them
+        if (lane == 0 && vt + BD_THREADS * k < n) l2_ask(a.w + vt + BD_THREADS * k);
     pdl_wait();
     pdl_go();
     const bool has_add = a.bo || a.moe.part;
+    float wv[BD_MAXC];
+#pragma unroll
+    for (int k = 0; k < BD_MAXC; ++k) wv[k] = a.w[min(vt + BD_THREADS * k, n - 1)];
     // ---- this GPU's addend of the row, this thread's columns.  The kernel is a chain of latencies, so everything a thread
     // reads (x, and a column's ten expert rows) is asked for before the first of it is used.
     float add[BD_MAXC], xo[BD_MAXC];

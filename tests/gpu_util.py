@@ -114,3 +114,14 @@ def run_gdn(c, want_y32=True):
     sync()
     return {"S": host(t["S"]), "hist": host(t["hist"]), "yq": host(yq).reshape(T, -1), "y32": host(y32) if want_y32 else None,
             "snap": host(snap), "hsnap": host(hsnap), "scratch_tail": host(scratch)[-nv:], "dev": (t, snap, hsnap)}
+
+
+def copy_last(dst, values, st, filler=1 << 26):
+    """Enqueues one fnx_copy_many job, a launch that lets the next one start early, whose last floats are `values`: returns
+    the tensor that will hold them (a view of dst, a float tensor of `filler` floats and theirs) and what must be kept."""
+    src = torch.zeros(filler + values.numel(), device=DEV)
+    src[filler:] = values.reshape(-1)
+    job = torch.frombuffer(bytearray(bytes(L.CopyJob(dst.data_ptr(), src.data_ptr(), src.numel() * 4))), dtype=torch.uint8).to(DEV)
+    sync()
+    L.call("fnx_copy_many", job.data_ptr(), 1, st)
+    return dst[filler:], (src, job)

@@ -43,6 +43,34 @@ def test_hc_read(T, n, hc, lr, fold, inject):
             assert np.array_equal(G.host(d_inj).view(np.uint32), inj.view(np.uint32)), "inject"
 
 
+@pytest.mark.parametrize("T,n,hc", [(1, 512, 4), (16, 3072, 4)])
+def test_hc_read_weights_written_by_the_launch_before(T, n, hc):
+    """The norm's weights may be what the launch directly ahead writes, one that lets its successor start early."""
+    import torch
+
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    c = cases.hc_case(T, n, hc, 64, seed=5, fold=False, inject=False)
+    st, filler = L.stream(), 1 << 26
+    dq, dd, uq, ud = G.dev(c["down"][0]), G.dev(c["down"][1]), G.dev(c["up"][0]), G.dev(c["up"][1])
+    wn = G.dev(c["w_norm"])
+    buf, scratch = torch.zeros(filler + wn.numel(), device=G.DEV), G.zeros(L.load().fnx_hc_scratch_floats(T, n, hc, 64))
+    R, got = G.dev(c["R"]), []
+
+    def read(w):
+        mixed = G.zeros((T, n))
+        L.call("fnx_hc_read", R.data_ptr(), None, None, w.data_ptr(), L.Q8S(dq.data_ptr(), dd.data_ptr()), L.Q8S(uq.data_ptr(), ud.data_ptr()),
+               None, c["eps"], mixed.data_ptr(), None, scratch.data_ptr(), None, T, n, hc, 64, st)
+        got.append(mixed)
+
+    read(wn)
+    w2, keep = G.copy_last(buf, wn, st, filler)
+    read(w2)
+    G.sync()
+    assert torch.equal(got[0].view(torch.int32), got[1].view(torch.int32))
+
+
 def test_hc_write():
     import oracle.binding as O
     from sfnx_b200 import lib as L

@@ -293,3 +293,25 @@ def test_boundary_rows_any_number_of_experts(topk, T, width):
     L.call("fnx_boundary_rows", x2.data_ptr(), None, C.byref(rows), None, wn.data_ptr(), y2.data_ptr(), q2.data_ptr(), T, width, 1e-6, err.data_ptr(), st)
     G.sync()
     assert torch.equal(x1.view(torch.int32), x2.view(torch.int32)) and torch.equal(y1.view(torch.int32), y2.view(torch.int32)) and torch.equal(q1, q2)
+
+
+@pytest.mark.parametrize("T,width", [(1, 512), (16, 3072), (3, 4096)])
+def test_boundary_weights_written_by_the_launch_before(T, width):
+    """The norm's weights may be what the launch directly ahead writes, one that lets its successor start early."""
+    import torch
+
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    st, filler = L.stream(), 1 << 26
+    g = torch.Generator("cuda").manual_seed(T)
+    x = torch.randn((T, width), generator=g, device=G.DEV)
+    wn = torch.randn(width, generator=g, device=G.DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=G.DEV)
+    x2, buf = x.clone(), torch.zeros(filler + width, device=G.DEV)
+    y1, y2 = G.zeros((T, width)), G.zeros((T, width))
+    L.call("fnx_rms_norm_rows", x.data_ptr(), None, wn.data_ptr(), y1.data_ptr(), None, T, width, 1e-6, st)
+    w2, keep = G.copy_last(buf, wn, st, filler)
+    L.call("fnx_boundary_rows", x2.data_ptr(), None, None, None, w2.data_ptr(), y2.data_ptr(), None, T, width, 1e-6, err.data_ptr(), st)
+    G.sync()
+    assert torch.equal(y1.view(torch.int32), y2.view(torch.int32))
