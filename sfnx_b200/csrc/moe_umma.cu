@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "copy_ring.h"
 #include "exact_math.cuh"
 #include "moe_internal.cuh"
 #include "umma.cuh"
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
     uint16_t* list = reinterpret_cast<uint16_t*>(raw + MU_RAW);
     static_assert(MU_COPY == 2 * MU_NS, "two copy warps a stage");
     static_assert(Raw::SLOTS * Raw::WIDTH * MU_BM <= MU_RAW, "the raw ring");
-    __shared__ __align__(8) unsigned long long full[MU_NS], empty[MU_NS], done[2], freed[2], rfull[Raw::SLOTS], rempty[Raw::SLOTS];
+    __shared__ __align__(8) unsigned long long full[MU_NS], empty[MU_NS], done[2], freed[2], idle, rfull[Raw::SLOTS], rempty[Raw::SLOTS];
     __shared__ unsigned tmem_base;
     __shared__ int ys[MU_COPY][MU_NMAX / 2];   // a copy warp's rows of x, -1: none
     if (tid == 0) {
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&done[s])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&freed[s])), "r"(MU_PROD / 32));
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&idle)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MU_PROD / 32) {   // all 512 columns of tensor memory: two results of 2 x 128 rows x (64 + 64)
@@ -282,6 +284,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
     const unsigned st_s = um_s32(stages);
     bool alive = true;   // false after a wait ran out
     unsigned g0 = 0, seq = 0, rc = 0;   // steps, tiles and raw loads that this role has behind it
+    CopyRing<Raw::SLOTS> ring;          // the loader's side of the raw loads
     const int nsteps = (nk + Raw::STEPS - 1) / Raw::STEPS;
     int run = 0;
     for (int base = 0; base < njobs; base += MU_LIST) {
@@ -375,17 +378,18 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
         } else if (warp == MU_PROD / 32 + 1) {
             // ---- the raw weights' loads, as far ahead as the ring holds, across the ends of tiles
             if (lane == 0) {
-                for (int it = first; it < items; it += stride) {
+                const auto landed = [&](unsigned s, unsigned parity) { return um_wait(&rfull[s], parity, a.fault); };
+                const auto used = [&](unsigned s, unsigned parity) { return um_wait(&rempty[s], parity, a.fault); };
+                for (int it = first; it < items && ring.alive; it += stride) {
                     const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
-                    for (int c = 0; c < nsteps; ++c, ++rc) {
-                        const unsigned slot = rc % Raw::SLOTS;
-                        if (rc >= Raw::SLOTS && alive) alive = um_wait(&rempty[slot], (rc / Raw::SLOTS - 1) & 1u, a.fault);
+                    for (int c = 0; c < nsteps && ring.acquire(used, landed); ++c) {
+                        const unsigned slot = ring.slot();
                         um_expect_tx(&rfull[slot], Raw::WIDTH * MU_BM);
                         um_tma3d(um_s32(raw + slot * (Raw::WIDTH * MU_BM)), &wmap, c * Raw::WIDTH, it % ntiles * MU_BM, expert, &rfull[slot]);
+                        ring.asked();
                     }
                 }
-                // no load is in flight when the block ends, also after a wait that ran out
-                for (unsigned k = rc < Raw::SLOTS ? 0 : rc - Raw::SLOTS; k < rc; ++k) um_wait(&rfull[k % Raw::SLOTS], (k / Raw::SLOTS) & 1u, a.fault);
+                ring.drain(landed);   // no load is in flight when the block ends
             }
         } else if (warp > MU_PROD / 32) {
             // ---- the activation rows, by asynchronous copies, two warps a step in turn: every stage's copies are issued side by side.  Lane i takes
@@ -447,17 +451,21 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
                                 um_mma(d, da + 2 * ks, db + 2 * ks, idesc, (unsigned) (k | ks));
                                 if (upper) um_mma(d + 128, da + 1024 + 2 * ks, db + 2 * ks, idesc, (unsigned) (k | ks));   // 128 rows on: 16 384 bytes
                             }
-                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&empty[s])) : "memory");
+                        um_commit(&empty[s]);
                     }
                     __syncwarp();
                 }
-                if (um_elect())
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&done[seq & 1u])) : "memory");
+                if (um_elect()) um_commit(&done[seq & 1u]);
                 __syncwarp();
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");   // only a wait that ran out leaves copies in flight here
         __syncthreads();   // the list may be rewritten
+    }
+    if (warp == MU_PROD / 32) {   // the results' readers waited for the MMAs, unless a wait of theirs ran out
+        if (um_elect()) um_commit(&idle);
+        __syncwarp();
+        um_wait(&idle, 0u, a.fault);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

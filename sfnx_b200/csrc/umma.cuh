@@ -26,6 +26,11 @@ __device__ __forceinline__ void um_mma(unsigned tmem, unsigned long long da, uns
                  : "memory");
 }
 
+// `bar` gets one arrival when every MMA that this thread has issued is done
+__device__ __forceinline__ void um_commit(unsigned long long* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(bar)) : "memory");
+}
+
 // One lane of a converged warp, the same one each time.  The branch it guards stays uniform for the compiler, so that
 // descriptors stay in uniform registers: under `lane == 0` each tcgen05.mma spent about 110 cycles moving them there.
 __device__ __forceinline__ bool um_elect() {
