@@ -17,18 +17,22 @@
 namespace fnxk {
 
 template <int SLOTS> struct CopyRing {
-    unsigned n = 0;      // copies asked for
-    bool alive = true;   // false after a wait ran out
-    FNX_RING_FN unsigned slot() const { return n % SLOTS; }
-    // Waits until copy n may be asked for; false: it must not.  empty(slot, parity), full(slot, parity): bounded waits,
-    // false when they run out.
+    unsigned slot = 0, round = 0;   // the next copy's; copies asked for: round SLOTS + slot
+    bool alive = true;              // false after a wait ran out
+    // Waits until the next copy may be asked for; false: it must not.  empty(slot, parity), full(slot, parity): bounded
+    // waits, false when they run out.  The copy before has landed by the time it has been read, so it is waited for first
+    // and costs nothing; asked for after the readers it was 1 % of a dense kernel's time.
     template <class Empty, class Full> FNX_RING_FN bool acquire(Empty empty, Full full) {
-        if (alive && n >= SLOTS) alive = empty(slot(), (n / SLOTS - 1) & 1u) && full(slot(), (n / SLOTS - 1) & 1u);
+        if (alive && round) alive = full(slot, (round - 1) & 1u) && empty(slot, (round - 1) & 1u);
         return alive;
     }
-    FNX_RING_FN void asked() { ++n; }
+    FNX_RING_FN void asked() {
+        if (++slot == SLOTS) slot = 0, ++round;
+    }
     template <class Full> FNX_RING_FN void drain(Full full) const {
-        for (unsigned k = n < SLOTS ? 0 : n - SLOTS; k < n; ++k) full(k % SLOTS, (k / SLOTS) & 1u);
+        for (unsigned s = 0; s < SLOTS; ++s)
+            if (s < slot) full(s, round & 1u);
+            else if (round) full(s, (round - 1) & 1u);
     }
 };
 

@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "copy_ring.h"
 #include "exact_math.cuh"
 #include "moe_internal.cuh"
 #include "umma.cuh"
@@ -51,9 +52,6 @@ __device__ __forceinline__ void du_mma_i8(unsigned tmem, unsigned long long da, 
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem), "l"(da), "l"(db),
                  "r"(idesc), "r"(0)   // p false: D = A B, nothing is accumulated across blocks
                  : "memory");
-}
-__device__ __forceinline__ void du_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(bar)) : "memory");
 }
 
 // two f32 in a 64-bit register, each half rounded as its scalar operation would be (Blackwell's packed f32 pipe)
@@ -101,7 +99,7 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
     unsigned char* b_op = a_st + (size_t) DU_STAGES * DU_ABYTES;               // [nkc][16 rows][128 bytes], swizzled
     uint16_t* dw_s = reinterpret_cast<uint16_t*>(b_op + (size_t) nkc * DU_BCHUNK);   // [2][nd][128][16] f16 block scales of a tile, swizzled in 32 bytes
     float* da_s = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(dw_s) + (size_t) 2 * DU_M * nd * 32);   // [nb][16]
-    __shared__ __align__(8) unsigned long long full_a[DU_STAGES], empty_a[DU_STAGES], tm_full[DU_SLOTS], tm_empty[DU_SLOTS], dw_full[2], dw_empty[2];
+    __shared__ __align__(8) unsigned long long full_a[DU_STAGES], empty_a[DU_STAGES], tm_full[DU_SLOTS], tm_empty[DU_SLOTS], dw_full[2], dw_empty[2], idle;
     __shared__ unsigned tmem_base;
     if (tid == 0) {
         for (int s = 0; s < DU_STAGES; ++s) {
@@ -116,6 +114,7 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&dw_full[s])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&dw_empty[s])), "r"(4 * ngrp));
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&idle)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == DU_EPI + 1) {   // all 512 columns of tensor memory: four groups of 2 x 4 x 16
@@ -130,21 +129,28 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
     if (warp == DU_EPI) {
         // ---- the TMA warp: weights do not wait for the kernel ahead
         if (lane == 0) {
-            int c = 0, tp = 0, nt = 0;
-            for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++nt, tp ^= 1) {
+            const auto w_landed = [&](unsigned s, unsigned parity) { return um_wait(&full_a[s], parity, a.fault); };
+            const auto w_used = [&](unsigned s, unsigned parity) { return um_wait(&empty_a[s], parity, a.fault); };
+            const auto d_landed = [&](unsigned s, unsigned parity) { return um_wait(&dw_full[s], parity, a.fault); };
+            const auto d_used = [&](unsigned s, unsigned parity) { return um_wait(&dw_empty[s], parity, a.fault); };
+            CopyRing<DU_STAGES> w_ring;   // weight tiles
+            CopyRing<2> d_ring;           // tiles' block scales
+            for (int tile = blockIdx.x; tile < a.ntiles && w_ring.alive && d_ring.acquire(d_used, d_landed); tile += gridDim.x) {
                 const DuTile t = du_tile(a, tile);
                 const CUtensorMap* mw = &maps.w[t.seg];
                 const CUtensorMap* md = &maps.d[t.seg];
-                if (nt >= 2 && alive) alive = um_wait(&dw_empty[tp], (unsigned) ((nt / 2 - 1) & 1), a.fault);
+                const unsigned tp = d_ring.slot;
                 um_expect_tx(&dw_full[tp], (unsigned) (a.H * nd * 32));
                 for (int i = 0; i < nd; ++i) um_tma2d(um_s32(dw_s) + (tp * nd + i) * DU_M * 32, md, 16 * i, t.row0, &dw_full[tp]);
-                for (int kc = 0; kc < nkc; ++kc, ++c) {
-                    const int s = c % DU_STAGES;
-                    if (c >= DU_STAGES && alive) alive = um_wait(&empty_a[s], (unsigned) ((c / DU_STAGES - 1) & 1), a.fault);
+                d_ring.asked();
+                for (int kc = 0; kc < nkc && w_ring.acquire(w_used, w_landed); ++kc) {
+                    const unsigned s = w_ring.slot;
                     um_expect_tx(&full_a[s], (unsigned) (a.H * DU_KC));
                     um_tma2d(a_s32 + s * DU_ABYTES, mw, kc * DU_KC, t.row0, &full_a[s]);
+                    w_ring.asked();
                 }
             }
+            w_ring.drain(w_landed), d_ring.drain(d_landed);   // no load is in flight when the block ends
         }
     } else {
         // ---- everyone else: the window's activations, once the kernel that makes them has finished
@@ -183,11 +189,15 @@ __global__ void __launch_bounds__(DU_THREADS, 1) k_q8s_umma(const __grid_constan
                         const unsigned long long da = um_desc(a_s32 + s * DU_ABYTES), db = um_desc(b_s32 + kc * DU_BCHUNK);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) du_mma_i8(tm + (unsigned) (slot * 128 + (c & 1) * 64 + 16 * j), da + 2 * j, db + 2 * j, idesc);
-                        du_commit(&empty_a[s]);
-                        if (c & 1) du_commit(&tm_full[slot]);   // tracks every MMA before it; the stages of a tile are even in number
+                        um_commit(&empty_a[s]);
+                        if (c & 1) um_commit(&tm_full[slot]);   // tracks every MMA before it; the stages of a tile are even in number
                     }
                     __syncwarp();
                 }
+            // the epilogue waited for the MMAs, unless a wait of its own ran out: tensor memory is freed after the last
+            if (um_elect()) um_commit(&idle);
+            __syncwarp();
+            um_wait(&idle, 0u, a.fault);
         } else if ((warp >> 2) < ngrp) {
             // ---- the epilogue warps
             const int q = warp & 3, g = warp >> 2, r_in = 32 * q + lane;

@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
                 for (int it = first; it < items && ring.alive; it += stride) {
                     const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
                     for (int c = 0; c < nsteps && ring.acquire(used, landed); ++c) {
-                        const unsigned slot = ring.slot();
+                        const unsigned slot = ring.slot;
                         um_expect_tx(&rfull[slot], Raw::WIDTH * MU_BM);
                         um_tma3d(um_s32(raw + slot * (Raw::WIDTH * MU_BM)), &wmap, c * Raw::WIDTH, it % ntiles * MU_BM, expert, &rfull[slot]);
                         ring.asked();

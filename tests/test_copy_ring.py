@@ -76,7 +76,7 @@ int main() {
         ring.drain(full);
         ring.drain(full);   // (a copy later than one wait: what is checked is that the ring waits for the right phases)
         for (int s = 0; s < SLOTS; ++s) m.bad += m.lands[s] >= 0;
-        if (m.stop == n && m.wild == n && seed %% 3 && ring.n != n) ++m.bad;   // nothing went wrong: every copy was asked for
+        if (m.stop == n && m.wild == n && seed %% 3 && ring.round * SLOTS + ring.slot != n) ++m.bad;   // nothing went wrong: every copy was asked for
         if (m.bad) return std::printf("seed %%u: %%ld\n", seed, m.bad), 1;
     }
     return 0;
