@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     unsigned char* Qlo = Qhi + A3_QBYTES;                       // each: 4 K-blocks x [96 rows x 128 B], swizzled
     unsigned char* KVst = Qlo + A3_QBYTES;                      // [3] 4 blocks of 64 dims x [64 rows x 128 B], swizzled: K(c), then V(c)
     unsigned char* Pst = KVst + A3_NBUF * A3_KBYTES;            // hi, lo: [96 rows x 128 B], 128-byte swizzle; then the pad
-    __shared__ __align__(8) unsigned long long mbar_s[2], mbar_o, kvbar[A3_NBUF], qbar;
+    __shared__ __align__(8) unsigned long long mbar_s[2], mbar_o, kvbar[A3_NBUF], qbar, idle;
     __shared__ unsigned tmem_base;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&mbar_s[0])));
@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&mbar_o)));
         for (int b = 0; b < A3_NBUF; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&kvbar[b])));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&qbar)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&idle)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     const bool copier = warp == 7;
     const int seg = lane;
     const size_t row_elems = (size_t) a.nkv * HD;
+    bool alive = true;   // false after a wait ran out; the copying warp then asks for nothing more
     // a buffer's mbarrier completes a phase per load: K(c) the even ones, V(c) the odd ones (waited for with parity 0, 1)
     auto tma_rows = [&](const CUtensorMap* map, int c, int b) {
         if (!copier || lane) return;
@@ -184,13 +186,16 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     // over them, for O += P(c) V(c); once those are done the K rows of chunk c + 3.  V(c) so has more than a chunk's time to
     // arrive and K(c + 3) most of one, with the memory two stages of each would take less one.
     const unsigned kv_s = um_s32(KVst);
+    int kq = 0, vq = 0;   // chunks whose K, whose V the copying warp has asked for (TMA)
     auto load_k = [&](int c) {
-        if (TMA) tma_rows(&maps.k, c_begin + c, c % A3_NBUF);
-        else load_rows(a.kc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
+        if (TMA) {
+            if (alive) tma_rows(&maps.k, c_begin + c, c % A3_NBUF), kq = c + 1;
+        } else load_rows(a.kc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
     };
     auto load_v = [&](int c) {
-        if (TMA) tma_rows(&maps.v, c_begin + c, c % A3_NBUF);
-        else load_rows(a.vc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
+        if (TMA) {
+            if (alive) tma_rows(&maps.v, c_begin + c, c % A3_NBUF), vq = c + 1;
+        } else load_rows(a.vc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
     };
     load_k(0);
     if (nc > 1) load_k(1);
@@ -234,7 +239,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
                 um_mma(tb, dh + oa, dk + ob, idesc_s, kb | ks);
                 um_mma(tb, dl + oa, dk + ob, idesc_s, 1u);
             }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&mbar_s[c & 1])) : "memory");
+        um_commit(&mbar_s[c & 1]);
     };
     auto issue_output = [&](int c) {   // O (+)= (Phi + Plo) V(c)
         const unsigned long long dv = um_desc_x(um_s32(KVst + (size_t) (c % A3_NBUF) * A3_KBYTES), A3_KBLK, 1024, 2);
@@ -244,7 +249,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
             um_mma(tm, dph + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, c | ks);
             um_mma(tm, dpl + (unsigned long long) (ks * 32 >> 4), dv + (unsigned long long) (ks * 16 * 128 >> 4), idesc_o, 1u);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_s32(&mbar_o)) : "memory");
+        um_commit(&mbar_o);
     };
     auto sync_all = [&] {   // stores and landed copies of every thread visible to the tensor core, tensor-memory accesses ordered
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -257,11 +262,13 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     tm = um_uniform(tmem_base);
     const bool issuer = warp == 3;   // one lane of it
     if (issuer) {
-        if (TMA) um_wait(&qbar, 0u, a.fault), um_wait(&kvbar[0], 0u, a.fault);   // the queries and K(0) have landed
+        if (TMA) {   // the queries and K(0) have landed
+            const bool ok = um_wait(&qbar, 0u, a.fault) && um_wait(&kvbar[0], 0u, a.fault);
+            alive = __all_sync(0xffffffffu, ok);
+        }
         if (um_elect()) issue_scores(0);
         __syncwarp();
     }
-    bool alive = true;   // false after a wait ran out
     auto copier_wait = [&](unsigned long long* bar, unsigned parity) {   // the copying warp alone waits for a set of MMAs
         bool ok = alive && um_wait(bar, parity, a.fault);
         ok = __all_sync(0xffffffffu, ok);
@@ -269,7 +276,8 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     };
     if (copier) {
-        copier_wait(&mbar_s[0], 0u);   // S(0) is complete: V(0) over K(0)
+        if (TMA) copier_wait(&kvbar[0], 0u);   // K(0) has landed, whatever its MMAs' issuer saw
+        copier_wait(&mbar_s[0], 0u);           // S(0) is complete: V(0) over K(0)
         load_v(0);
     }
     asm volatile("cp.async.commit_group;");
@@ -277,7 +285,10 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     for (int i = 0; i < nc; ++i) {
         const int buf = i & 1;
         if (issuer && i + 1 < nc) {   // the next chunk's scores while this chunk's are used
-            if (TMA) um_wait(&kvbar[(i + 1) % A3_NBUF], 0u, a.fault);   // K(i + 1) has landed
+            if (TMA && alive) {   // K(i + 1) has landed
+                const bool ok = um_wait(&kvbar[(i + 1) % A3_NBUF], 0u, a.fault);
+                alive = __all_sync(0xffffffffu, ok);
+            }
             if (um_elect()) issue_scores(i + 1);
             __syncwarp();
         }
@@ -336,6 +347,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         if (i > 0 && i + 2 < nc) load_k(i + 2);   // over V(i - 1), whose MMAs are done
         asm volatile("cp.async.commit_group;");
         if (copier && i + 1 < nc) {
+            if (TMA) copier_wait(&kvbar[(i + 1) % A3_NBUF], 0u);
             copier_wait(&mbar_s[buf ^ 1], (unsigned) (((i + 1) >> 1) & 1));   // S(i + 1) is complete: V(i + 1) over K(i + 1)
             load_v(i + 1);
         }
@@ -414,6 +426,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     {
         bool ok = alive && um_wait(&mbar_o, (nc - 1) & 1, a.fault);
         ok = __all_sync(0xffffffffu, ok);
+        alive = alive && ok;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (worker) {
 #pragma unroll 1
@@ -442,6 +455,17 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // Nothing is in flight when the block ends, also after a wait that ran out.  A load over another was asked for only when
+    // that one had landed, so the buffers' last loads are what is left: V(c) where it was asked for, else K(c)
+    if (TMA && copier) {
+        um_wait(&qbar, 0u, a.fault);
+        for (int c = max(kq - A3_NBUF, 0); c < kq; ++c) um_wait(&kvbar[c % A3_NBUF], c < vq ? 1u : 0u, a.fault);
+    }
+    if (issuer && !alive) {   // (alive: the wait for mbar_o above was for the last MMAs)
+        if (um_elect()) um_commit(&idle);
+        __syncwarp();
+        um_wait(&idle, 0u, a.fault);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
