@@ -552,9 +552,12 @@ __global__ void __launch_bounds__(AX_THREADS) k_attn_cells(const float* __restri
             row_s[i] = r;
             um_bulk(um_s32(k_s + (size_t) i * KLD), kc + r, HD * 2, &kbar);
         }
-        um_wait(&kbar, kphase, fault);
+        const bool landed = um_wait(&kbar, kphase, fault);
+        if (!__syncthreads_and(landed)) {   // (row_s is complete for the values) a wait ran out: nothing more is asked for,
+            um_wait(&kbar, kphase, fault);   // and the block does not end under the copies
+            break;
+        }
         kphase ^= 1u;
-        __syncthreads();   // (row_s is complete for the values)
         // ---- scores of chunk `warp`
         float sv[QM];
         const int at = warp * ATT_CH + lane;
