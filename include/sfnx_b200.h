@@ -482,7 +482,7 @@ int fnx_draft_begin(const FnxStackCfg* cfg, const FnxDraft* d, void* ws, const f
 enum { FNX_AFTER_NONE = 0, FNX_AFTER_SUM_BO = 1, FNX_AFTER_GATHER_PARTIALS = 2, FNX_AFTER_GATHER_BEST = 3 };
 /* workspace buffers a caller reads or writes */
 enum { FNX_BUF_X = 0, FNX_BUF_BO = 1, FNX_BUF_PARTIALS = 2, FNX_BUF_BEST_V = 3, FNX_BUF_BEST_I = 4, FNX_BUF_ERR = 5, FNX_BUF_CTL = 6,
-       FNX_BUF_LOGITS = 7, FNX_BUF_COPY_JOBS = 8, FNX_BUF_NJOBS = 9,
+       FNX_BUF_LOGITS = 7, FNX_BUF_COPY_JOBS = 8 /* retired: no such buffer */, FNX_BUF_NJOBS = 9,
        FNX_BUF_STREAMS = 10 /* hc > 1: the residual streams [T][hc n] as the window left them (a draft layer's source rows) */ };
 
 size_t fnx_window_workspace_bytes(const FnxStackCfg* cfg);
@@ -496,7 +496,8 @@ int fnx_window_stage(const FnxStackCfg* cfg, const FnxLayer* layers, const FnxHe
 void* fnx_window_buf(const FnxStackCfg* cfg, void* ws, int which);
 /* keep the first n of the last window's T rows (reference Engine::commit, src/engine_common.cu:525-568): per DeltaNet
  * layer S <- snap[n-1] and the written history half <- hsnap[n-1]; tag is the window's tag (its parity names the
- * half).  host_jobs: pinned host memory for nlayers * (2 FnxCopyJob + 1 FnxGdnReplay), copied into the workspace */
+ * half).  host_jobs: host memory for nlayers * (2 FnxCopyJob + 1 FnxGdnReplay) that the call writes its job table to; the table
+ * goes with the launches, so the memory is free again when the call returns and need not be pinned */
 int fnx_window_commit(const FnxStackCfg* cfg, const FnxLayer* layers, void* ws, int T, int n, int tag, void* host_jobs, void* st);
 
 /* a second stream for work that does not depend on its neighbours (the shared expert beside the routed experts, the
@@ -536,7 +537,8 @@ typedef struct FnxWindowLanes {
 } FnxWindowLanes;
 int fnx_window_stage_lanes(const FnxStackCfg* cfg, const FnxLayer* layers, const FnxHead* head, void* ws, const FnxWindowLanes* lanes, int stage,
                            void* st);
-/* keeps the first n[s] rows of lane s (tags[s]: the lane's window tag, whose low bit says which history half was read) */
+/* keeps the first n[s] rows of lane s (tags[s]: the lane's window tag, whose low bit says which history half was read).
+ * host_jobs: as fnx_window_commit's, for nlayers * 2 * nseg FnxCopyJob */
 int fnx_window_commit_lanes(const FnxStackCfg* cfg, const FnxLayer* layers, void* ws, const FnxWindowLanes* lanes, const int* n, const int* tags,
                             void* host_jobs, void* st);
 

@@ -86,7 +86,7 @@ struct Traced {
 // the workspace's buffers, as offsets from its base
 struct Ws {
     size_t x, bo, xn, xq, qkvz, ab, yq, qg, k, v, att, partials, att_scratch, rlogits, topi, topw, jobs_gu, jobs_dn, njobs, rscratch, gu,
-        hq, part, sh_gu, shq, sh, logits, keys, best_v, best_i, err, ctl, gdn_scratch, copy_jobs, hc_R, hc_inj, hc_scratch, dr_en, dr_e2, dr_h2, dr_q, qsa_y, qsa_q, qsa_scores, qsa_cells, qsa_ncells, total;
+        hq, part, sh_gu, shq, sh, logits, keys, best_v, best_i, err, ctl, gdn_scratch, hc_R, hc_inj, hc_scratch, dr_en, dr_e2, dr_h2, dr_q, qsa_y, qsa_q, qsa_scores, qsa_cells, qsa_ncells, total;
 };
 
 static Ws carve(const FnxStackCfg& c) {
@@ -133,7 +133,6 @@ static Ws carve(const FnxStackCfg& c) {
     w.err = take(16);
     w.ctl = take(16);
     w.gdn_scratch = take(fnx_gdn_scratch_floats(c.nv) * 4);
-    w.copy_jobs = take((size_t) c.nlayers * 2 * FNX_MAXT * sizeof(FnxCopyJob));   // up to a lane a row
     const size_t hcn = c.hc > 1 ? (size_t) c.hc : 0;   // hyper-connections: the residual streams, the two halves' inject values, the read's scratch
     w.hc_R = take(T * hcn * n * 4);
     w.hc_inj = take(2 * T * (hcn ? hcn : 1) * 4);
@@ -227,7 +226,6 @@ void* fnx_window_buf(const FnxStackCfg* cfg, void* ws, int which) {
         case FNX_BUF_ERR: return b + w.err;
         case FNX_BUF_CTL: return b + w.ctl;
         case FNX_BUF_LOGITS: return b + w.logits;
-        case FNX_BUF_COPY_JOBS: return b + w.copy_jobs;
         case FNX_BUF_NJOBS: return b + w.njobs;
         case FNX_BUF_STREAMS: return b + w.hc_R;
     }

@@ -478,8 +478,8 @@ class WindowRunner:
         assert 0 < self.nstages <= 1024, lib.fnx_last_error()
         self.after = list(after[: self.nstages])
         self.job_bytes = len(s.kinds) * (2 * C.sizeof(L.CopyJob) + C.sizeof(L.GdnReplay))
-        self.h_jobs = torch.zeros(64 * self.job_bytes, dtype=torch.uint8).pin_memory()   # a ring of job tables
-        self.commits = 0
+        # where a commit writes its job table, free again when it returns
+        self.h_jobs = torch.zeros(self.job_bytes if lanes is None else len(s.kinds) * 2 * L.MAXT * C.sizeof(L.CopyJob), dtype=torch.uint8)
         self.launches = 0
         self.graph = self.graph_io = None
         # a side stream for the window's independent branches (the library forks and joins with these events)
@@ -679,11 +679,9 @@ class WindowRunner:
         """Keep the first n[i] rows of lane i of the last window."""
         ln = self.lanes
         nn, tt = (C.c_int * ln.nseg)(*n), (C.c_int * ln.nseg)(*tags)
-        jobs = torch.zeros(len(self.stack.shape.kinds) * 2 * L.MAXT * C.sizeof(L.CopyJob), dtype=torch.uint8).pin_memory()
-        with torch.cuda.stream(self.stream):
-            L.call("fnx_window_commit_lanes", C.byref(self.stack.cfg), self.stack.layers, self.stack.ws.data_ptr(), C.byref(ln.c), nn, tt,
-                   jobs.data_ptr(), torch.cuda.current_stream().cuda_stream)
-        self.stream.synchronize()   # the job table is read by an asynchronous copy
+        L.call("fnx_window_commit_lanes", C.byref(self.stack.cfg), self.stack.layers, self.stack.ws.data_ptr(), C.byref(ln.c), nn, tt,
+               self.h_jobs.data_ptr(), self.stream.cuda_stream)
+        torch.cuda.current_stream().wait_stream(self.stream)   # what the caller enqueues next sees the lanes rolled back
 
     def merge_best(self):
         if self.stack.ncard == 1:
@@ -714,12 +712,8 @@ class WindowRunner:
         replay log the states advance only here, also when every row is kept)."""
         if n >= self.T and not self.stack.gdn_log:
             return
-        slot = self.commits % 64   # the table is read by an asynchronous copy: a slot is reused only 64 commits later
-        self.commits += 1
-        if slot == 0 and self.commits > 1:
-            self.stream.synchronize()
         L.call("fnx_window_commit", C.byref(self.stack.cfg), self.stack.layers, self.stack.ws.data_ptr(), self.T, n, tag,
-               self.h_jobs.data_ptr() + slot * self.job_bytes, self.stream.cuda_stream)
+               self.h_jobs.data_ptr(), self.stream.cuda_stream)
 
     def close(self):
         """Releases what must go before the process group does: the captured graph (its NCCL nodes hold the communicator)

@@ -465,3 +465,43 @@ def test_commit_tables_of_any_length(nlayers, n, log):
     L.call("fnx_window_commit", C.byref(cfg), layers, ws.data_ptr(), T, n, tag, host.data_ptr(), L.stream())
     torch.cuda.synchronize()
     assert torch.equal(hist, want_hist) and torch.equal(S, want_S)
+
+
+def test_commits_neither_wait_nor_keep_the_table():
+    """The rollback's job table goes with its launches: the calls return while the GPU is still busy ahead of them, the
+    table may be written over at once, and work that the caller enqueues after commit_lanes sees the lanes rolled back."""
+    import torch
+
+    from sfnx_b200.window import LaneSet, StackShape, SyntheticStack, WindowRunner
+
+    shape = StackShape(n=512, nexp=32, topk=4, ff=128, nkh=2, nvh=4, nq=8, nkv=2, hd=256, nrot=64, vocab=512, kinds=[0, 1, 0], ctx=600, kv_slack=64)
+    stack = SyntheticStack(shape, seed=21, device="cuda:0", gdn_log=False)
+    lanes = LaneSet(stack, 2, 3)
+    runner = WindowRunner(stack, 6, lanes=lanes)
+    rng = np.random.default_rng(22)
+    S0, h0 = ({l: [t.clone() for t in ts] for l, ts in d.items()} for d in (lanes.S, lanes.hist))
+    ids = [int(v) for v in rng.integers(0, shape.vocab, 6)]
+
+    def once(busy):
+        for l in S0:
+            for i in range(2):
+                lanes.S[l][i].copy_(S0[l][i])
+                lanes.hist[l][i].copy_(h0[l][i])
+        torch.cuda.synchronize()
+        runner.window_lanes(ids, [40, 90], [1, 2])
+        if busy:
+            with torch.cuda.stream(runner.stream):
+                torch.cuda._sleep(200_000_000)
+        runner.commit_lanes([1, 2], [1, 2])
+        waiting = not runner.stream.query()
+        runner.h_jobs.fill_(255)
+        return waiting, [t.clone() for d in (lanes.S, lanes.hist) for l in sorted(d) for t in d[l]]   # on the caller's stream
+
+    once(False)
+    torch.cuda.synchronize()
+    _, want = once(False)
+    torch.cuda.synchronize()
+    waiting, got = once(True)
+    assert waiting, "commit_lanes waited for the GPU"
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
