@@ -657,9 +657,8 @@ class WindowRunner:
             tok = self.window([token], pos0 + i, tag)[0]
             out.append(tok)
             token = tok
-            if i + 1 < k:
-                with torch.cuda.stream(self.stream):
-                    self.src[0].copy_(streams)
+            with torch.cuda.stream(self.stream):
+                self.src[0].copy_(streams)   # after the last step too: a window() call then goes on with the chain
         return out
 
     def window_lanes(self, rows, pos, tags):

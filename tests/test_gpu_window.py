@@ -260,6 +260,11 @@ def test_draft_chain_equals_the_oracles(monkeypatch):
         tok, src = best[0], orc.last_R[0].copy()
     got = r1.draft_chain(torch.from_numpy(src0).to(stack.dev), 5, shape.ctx, 4, 1)
     assert got == want
+    logits = r1.logits.clone()
+    # a chain of three, and the fourth step as a window of its own: the runner's source row is the chain's newest stream
+    got = r1.draft_chain(torch.from_numpy(src0).to(stack.dev), 5, shape.ctx, 3, 1)
+    assert got + r1.window([got[-1]], shape.ctx + 3, 1) == want
+    assert torch.equal(logits.view(torch.int32), r1.logits.view(torch.int32))
 
 
 def test_window_int8_kv_bit_exact():
