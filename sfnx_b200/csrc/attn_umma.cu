@@ -155,10 +155,13 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     const int seg = lane;
     const size_t row_elems = (size_t) a.nkv * HD;
     bool alive = true;   // false after a wait ran out; the copying warp then asks for nothing more
-    // a buffer's mbarrier completes a phase per load: K(c) the even ones, V(c) the odd ones (waited for with parity 0, 1)
+    unsigned loads = 0;   // the copying lane's: bit b is set after an odd number of loads into buffer b
+    // a buffer's mbarrier completes a phase per load: K(c) the even ones, V(c) the odd ones (waited for with parity 0, 1).
+    // `alive` is looked at by the copying lane alone: a look by every warp cost 3 % of a scan (32 768 positions 52.7 -> 54.5 us)
     auto tma_rows = [&](const CUtensorMap* map, int c, int b) {
-        if (!copier || lane) return;
+        if (!copier || lane || !alive) return;
         um_expect_tx(&kvbar[b], A3_KBYTES);
+        loads ^= 1u << b;
 #pragma unroll
         for (int blk = 0; blk < 4; ++blk)
             um_tma2d(um_s32(KVst) + b * A3_KBYTES + blk * A3_KBLK, map, kvl * HD + blk * 64, c * A3_CH, &kvbar[b]);
@@ -186,16 +189,13 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     // over them, for O += P(c) V(c); once those are done the K rows of chunk c + 3.  V(c) so has more than a chunk's time to
     // arrive and K(c + 3) most of one, with the memory two stages of each would take less one.
     const unsigned kv_s = um_s32(KVst);
-    int kq = 0, vq = 0;   // chunks whose K, whose V the copying warp has asked for (TMA)
     auto load_k = [&](int c) {
-        if (TMA) {
-            if (alive) tma_rows(&maps.k, c_begin + c, c % A3_NBUF), kq = c + 1;
-        } else load_rows(a.kc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
+        if (TMA) tma_rows(&maps.k, c_begin + c, c % A3_NBUF);
+        else load_rows(a.kc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
     };
     auto load_v = [&](int c) {
-        if (TMA) {
-            if (alive) tma_rows(&maps.v, c_begin + c, c % A3_NBUF), vq = c + 1;
-        } else load_rows(a.vc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
+        if (TMA) tma_rows(&maps.v, c_begin + c, c % A3_NBUF);
+        else load_rows(a.vc, c_begin + c, kv_s + (c % A3_NBUF) * A3_KBYTES);
     };
     load_k(0);
     if (nc > 1) load_k(1);
@@ -262,10 +262,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     tm = um_uniform(tmem_base);
     const bool issuer = warp == 3;   // one lane of it
     if (issuer) {
-        if (TMA) {   // the queries and K(0) have landed
-            const bool ok = um_wait(&qbar, 0u, a.fault) && um_wait(&kvbar[0], 0u, a.fault);
-            alive = __all_sync(0xffffffffu, ok);
-        }
+        if (TMA) alive = um_wait(&qbar, 0u, a.fault) && um_wait(&kvbar[0], 0u, a.fault);   // the queries and K(0) have landed
         if (um_elect()) issue_scores(0);
         __syncwarp();
     }
@@ -285,10 +282,7 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     for (int i = 0; i < nc; ++i) {
         const int buf = i & 1;
         if (issuer && i + 1 < nc) {   // the next chunk's scores while this chunk's are used
-            if (TMA && alive) {   // K(i + 1) has landed
-                const bool ok = um_wait(&kvbar[(i + 1) % A3_NBUF], 0u, a.fault);
-                alive = __all_sync(0xffffffffu, ok);
-            }
+            if (TMA && alive) alive = um_wait(&kvbar[(i + 1) % A3_NBUF], 0u, a.fault);   // K(i + 1) has landed
             if (um_elect()) issue_scores(i + 1);
             __syncwarp();
         }
@@ -456,10 +450,10 @@ __global__ void __launch_bounds__(AU_THREADS) k_attn_umma(const __grid_constant_
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     // Nothing is in flight when the block ends, also after a wait that ran out.  A load over another was asked for only when
-    // that one had landed, so the buffers' last loads are what is left: V(c) where it was asked for, else K(c)
-    if (TMA && copier) {
+    // that one had landed, so a wait for a buffer's last load is left (a buffer without any: its phase -1 counts as done)
+    if (TMA && copier && lane == 0) {
         um_wait(&qbar, 0u, a.fault);
-        for (int c = max(kq - A3_NBUF, 0); c < kq; ++c) um_wait(&kvbar[c % A3_NBUF], c < vq ? 1u : 0u, a.fault);
+        for (int b = 0; b < A3_NBUF; ++b) um_wait(&kvbar[b], (loads >> b & 1u) ^ 1u, a.fault);
     }
     if (issuer && !alive) {   // (alive: the wait for mbar_o above was for the last MMAs)
         if (um_elect()) um_commit(&idle);
