@@ -481,7 +481,7 @@ class WindowRunner:
         # where a commit writes its job table, free again when it returns
         self.h_jobs = torch.zeros(self.job_bytes if lanes is None else len(s.kinds) * 2 * L.MAXT * C.sizeof(L.CopyJob), dtype=torch.uint8)
         self.launches = 0
-        self.graph = self.graph_io = None
+        self.graph = self.graph_io = self.graph_chain = None
         # a side stream for the window's independent branches (the library forks and joins with these events)
         self.side = torch.cuda.Stream() if overlap else None
         self.ev_fork, self.ev_join = torch.cuda.Event(), torch.cuda.Event()
@@ -503,6 +503,14 @@ class WindowRunner:
                         self._enqueue()
                         self._read_back()
                     self.graph_io = g
+                    if s.draft and T == 1:   # a chain's step: its streams become the runner's source row too
+                        g = torch.cuda.CUDAGraph()
+                        with torch.cuda.graph(g, stream=self.stream):
+                            self._upload()
+                            self._enqueue()
+                            self._read_back()
+                            self._chain()
+                        self.graph_chain = g
         torch.cuda.synchronize()
 
     def _make_ring(self, count):
@@ -605,6 +613,9 @@ class WindowRunner:
             self.h_cv.copy_(self.all_cv, non_blocking=True)
             self.h_ci.copy_(self.all_ci, non_blocking=True)
 
+    def _chain(self):
+        self.src[0].copy_(self.stack.buf(10, torch.float32, self.stack.shape.hc * self.stack.shape.n))
+
     def launch(self):
         """Enqueues one window on the runner's stream (the caller has set ids and ctl)."""
         with torch.cuda.stream(self.stream):
@@ -616,23 +627,30 @@ class WindowRunner:
     def window(self, rows, pos0, tag):
         """One window from host token ids: uploads ids and (position, tag), runs, reads back every row's argmax (merged
         across GPUs: the lower GPU wins a tie) and the error word.  Returns the argmax tokens as a list."""
+        self._host_in(rows, pos0, tag)
+        return self._run()
+
+    def _host_in(self, rows, pos0, tag):
         T = self.T
         if pos0 + T > self.stack.shape.ctx + self.stack.shape.kv_slack:
             raise L.FnxError("window at position %d + %d rows is past the K/V cache (%d positions)" %
                              (pos0, T, self.stack.shape.ctx + self.stack.shape.kv_slack))
         self.h_in_np[:T] = rows
         self.h_in_np[L.MAXT], self.h_in_np[L.MAXT + 1] = pos0, tag
-        return self._run()
 
-    def _run(self):
-        """Uploads the host's ids and control words, runs the window, reads the result back and merges it."""
+    def _run(self, chain=False):
+        """Uploads the host's ids and control words, runs the window, reads the result back and merges it; chain: and makes
+        the streams it leaves the runner's source row."""
+        graph = self.graph_chain if chain else self.graph_io
         with torch.cuda.stream(self.stream):
-            if self.graph_io is not None:
-                self.graph_io.replay()
+            if graph is not None:
+                graph.replay()
             else:
                 self._upload()
                 self.launch()
                 self._read_back()
+                if chain:
+                    self._chain()
         self.stream.synchronize()
         err = int(self.h_err[0])
         if err != 0:
@@ -649,16 +667,13 @@ class WindowRunner:
         layer's own streams as its last window left them; each step's token = the step before's argmax).  src_row:
         [hc n] floats on the device; returns the k drafted head rows (indices into the draft vocabulary)."""
         assert self.stack.shape.draft and self.T == 1, "a draft layer's runner of one row"
-        streams = self.stack.buf(10, torch.float32, self.stack.shape.hc * self.stack.shape.n)
         out = []
         with torch.cuda.stream(self.stream):
             self.src[0].copy_(src_row.reshape(-1))
         for i in range(k):
-            tok = self.window([token], pos0 + i, tag)[0]
-            out.append(tok)
-            token = tok
-            with torch.cuda.stream(self.stream):
-                self.src[0].copy_(streams)   # after the last step too: a window() call then goes on with the chain
+            self._host_in([token], pos0 + i, tag)
+            token = self._run(chain=True)[0]   # after the last step too: a window() call then goes on with the chain
+            out.append(token)
         return out
 
     def window_lanes(self, rows, pos, tags):
@@ -718,7 +733,7 @@ class WindowRunner:
         """Releases what must go before the process group does: the captured graph (its NCCL nodes hold the communicator)
         and the peer-mapped buffers of the sum across GPUs."""
         torch.cuda.synchronize()
-        self.graph = self.graph_io = None
+        self.graph = self.graph_io = self.graph_chain = None
         self.ring = None
         self.ring_keep = None
         torch.cuda.synchronize()
