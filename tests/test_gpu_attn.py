@@ -181,6 +181,65 @@ def test_attention_rows_of_several_sequences():
     assert np.array_equal(G.host(part).view(np.uint32), ref.view(np.uint32))
 
 
+def _int8_pages(c, ref, rpp, spare):
+    """An int8 cache's rows (after the window's append) cut into pages of rpp rows: [pages][spare + halves a page]."""
+    from sfnx_b200 import lib as L
+
+    nkv, hd, rows = c["nkv"], c["hd"], c["q8_rows"]
+    page = L.load().fnx_kvq_halves(rpp, nkv, hd)
+    out = []
+    for cache in (ref["kc"][0], ref["vc"][0]):
+        q, d = cache[:rows * nkv * hd // 2].reshape(rows, -1), cache[rows * nkv * hd // 2:].reshape(rows, -1)
+        pages = np.zeros(((rows + rpp - 1) // rpp, page + spare), np.uint16)
+        for j, pg in enumerate(pages):
+            qj, dj = q[j * rpp:(j + 1) * rpp].reshape(-1), d[j * rpp:(j + 1) * rpp].reshape(-1)
+            pg[:qj.size] = qj
+            pg[rpp * nkv * hd // 2:rpp * nkv * hd // 2 + dj.size] = dj
+        out.append(pages)
+    return out
+
+
+@pytest.mark.parametrize("hd,nq,nkv,rpp,spare", [(256, 24, 4, 64, 0), (256, 6, 1, 20, 4), (128, 12, 2, 12, 0), (128, 3, 1, 4, 4)])
+def test_attention_int8_rows_behind_page_tables(hd, nq, nkv, rpp, spare):
+    """int8 rows on pages (values, then scales; a page may begin on any 8-byte boundary): windows of one sequence, one and
+    sixteen rows, and six rows of three sequences, bit for bit."""
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    lanes = [(2, 300, 81), (1, 37, 82), (3, 700, 83), (16, 410, 84), (1, 90, 85)]
+    cs = [cases.attn_case_q8(cases.attn_case(T=T, ctx=ctx, nq=nq, nkv=nkv, hd=hd, seed=seed)) for T, ctx, seed in lanes]
+    refs = [cases.attn_oracle(c) for c in cs]
+    pages = [_int8_pages(c, r, rpp, spare) for c, r in zip(cs, refs)]
+    rng = np.random.default_rng(86)
+    phys = rng.permutation(sum(len(k) for k, _ in pages) + 3).astype(np.int32)
+    pool = np.zeros((2, len(phys), pages[0][0].shape[1]), np.uint16)
+    pts, at = [], 0
+    for kp, vp in pages:
+        pt = phys[at:at + len(kp)]
+        at += len(kp)
+        pool[0][pt], pool[1][pt] = kp, vp
+        pts.append(G.dev(pt))
+    kc, vc, st = G.dev(pool[0]), G.dev(pool[1]), L.stream()
+    page = pool.shape[2]
+    for c, r, pt in zip(cs, refs, pts):   # a sequence alone
+        T, qg, pos = c["T"], G.dev(r["qg"]), G.dev(np.array([c["pos0"]], np.int32))
+        part, scratch = G.zeros((T, nq, hd + 2)), G.zeros(L.load().fnx_attn_scratch_floats(nq, hd, T))
+        L.call("fnx_attn_partial_exact", qg.data_ptr(), kc.data_ptr(), vc.data_ptr(), L.KvPages(pt.data_ptr(), page, rpp, 0, 1), part.data_ptr(), 0, 1,
+               T, pos.data_ptr(), nq, nkv, hd, scratch.data_ptr(), st)
+        G.sync()
+        assert np.array_equal(G.host(part).view(np.uint32), r["part"][0].view(np.uint32)), T
+    rows = [(i, t) for i, (T, _, _) in enumerate(lanes[:3]) for t in range(T)]   # three together
+    pos = [G.dev(np.array([lanes[i][1] + t], np.int32)) for i, t in rows]
+    ppos = G.dev(np.array([p.data_ptr() for p in pos], np.uint64))
+    ppt = G.dev(np.array([pts[i].data_ptr() for i, _ in rows], np.uint64))
+    qg = G.dev(np.concatenate([r["qg"] for r in refs[:3]]))
+    part, scratch = G.zeros((len(rows), nq, hd + 2)), G.zeros(L.load().fnx_attn_scratch_floats(nq, hd, len(rows)))
+    L.call("fnx_attn_part_lanes", qg.data_ptr(), kc.data_ptr(), vc.data_ptr(), L.KvPages(None, page, rpp, 0, 1), L.LaneRows(ppos.data_ptr(), ppt.data_ptr()),
+           part.data_ptr(), 0, 1, len(rows), nq, nkv, hd, scratch.data_ptr(), st)
+    G.sync()
+    assert np.array_equal(G.host(part).view(np.uint32), np.concatenate([r["part"][0] for r in refs[:3]]).view(np.uint32))
+
+
 def test_attention_scan_timings(capsys):
     """Device times of the three scans of one layer at the benchmark's shape (T = 16, 24 / 4 heads of 256, 32 768 positions on
     one GPU): the tcgen05 scan over f16 rows, the exact-order scan over f16 rows and over int8 rows.  Printed; no bound

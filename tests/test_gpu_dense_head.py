@@ -175,3 +175,22 @@ def test_l2_prefetch_changes_nothing():
         lib.call("fnx_l2_prefetch", x.data_ptr() + off, n, st)
     torch.cuda.synchronize()
     assert torch.equal(x, ref)
+
+
+@pytest.mark.parametrize("rows,n,add", [(1, 12288, False), (3, 12288, True), (2, 12320, True), (1, 16384, False), (2, 32, True), (16, 1056, True)])
+def test_rms_norm_rows_of_any_width(oracle, rows, n, add):
+    """Rows narrower than a block, and rows of many columns a thread."""
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+    import torch
+
+    rng = np.random.default_rng(n + rows)
+    x, a, wn = (rng.standard_normal(k).astype(np.float32) for k in ((rows, n), (rows, n), (n,)))
+    dx, da, dw, y, q = G.dev(x), G.dev(a), G.dev(wn), G.zeros((rows, n)), G.zeros(rows * (n // 32) * 36, torch.uint8)
+    L.call("fnx_rms_norm_rows", dx.data_ptr(), da.data_ptr() if add else None, dw.data_ptr(), y.data_ptr(), q.data_ptr(), rows, n, 1e-6, L.stream())
+    G.sync()
+    x2 = (x + a).astype(np.float32) if add else x
+    assert np.array_equal(G.host(dx), x2)
+    ref = oracle.rms_norm_rows(x2, wn, 1e-6)
+    assert np.array_equal(G.host(y).view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(G.host(q).reshape(rows, -1), oracle.quantize_q8_1(ref).view(np.uint8).reshape(rows, -1))

@@ -176,3 +176,50 @@ def test_no_job_past_the_capacity(cap, count):
     ref, mag = O.moe_mma(_weights16(w, "gu"), jobs[:cap], cap, x16, rows, count)
     _close(got[:cap], ref[:cap], mag[:cap], n)
     assert np.isnan(got[cap:]).all()
+
+
+@pytest.mark.parametrize("kind,n,ffs", [("q4k", 768, 288), ("q4k", 256, 288), ("q8_0", 800, 288), ("q8_0", 736, 96)])
+def test_many_tiles_a_block(kind, n, ffs):
+    """Three and more tiles for every block of the persistent kernel, gate|up and down: matrices of two and a half to four tiles
+    of rows, jobs of 1 to 64 rows alone and in pairs (64 + 64 among them), one to thirteen steps with and without a last one
+    of 32 columns.  What is carried from tile to tile (the raw ring, the scales asked for ahead, the two results in tensor
+    memory) shows in the sums."""
+    from oracle import binding as O
+
+    nexp, sizes = 7, ([1], [17], [64], [2], [64, 64], [3, 9], [5])
+    w = (cases.moe_weights if kind == "q4k" else cases.moe_weights_q8)(n=n, nexp=nexp, ffs=ffs, seed=44)
+    rng = np.random.default_rng(45)
+    for which, rows, cols in (("gu", 2 * ffs, n), ("dn", n, ffs)):
+        tiles = (rows + 255) // 256
+        pairs = (3 * 160 + tiles - 1) // tiles
+        take = [(g % nexp, k) for g in range(pairs) for k in sizes[g % len(sizes)]]
+        jobs, P = np.zeros(len(take), O.BIGJOB_DTYPE), 0
+        x16 = _f16_bits(rng.standard_normal((131, cols)))
+        for jb, (e, k) in zip(jobs, take):
+            jb["w"], jb["n"] = e, k
+            jb["y"][:k], jb["out"][:k] = rng.integers(0, 131, k), np.arange(P, P + k)
+            P += k
+        ex, keep = _experts(w, which)
+        got = _run("fnx_moe_gate_up_mma" if which == "gu" else "fnx_moe_down_mma", ex, jobs, x16, P)
+        ref, mag = O.moe_mma(_weights16(w, which), jobs, len(jobs), x16, rows, P)
+        _close(got, ref, mag, cols)
+
+
+@pytest.mark.parametrize("P,ffs,off", [(1, 5, 0), (7, 33, 0), (40, 12, 0), (3, 64, 1), (1, 8, 2), (513, 96, 3)])
+def test_swiglu_of_any_width_and_address(P, ffs, off):
+    """Widths that are no whole 16-byte pieces and arrays that begin off a 16-byte boundary (the value-a-thread kernel)."""
+    import torch
+
+    from oracle import binding as O
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    gu = (3 * np.random.default_rng(ffs).standard_normal((P, 2 * ffs))).astype(np.float32)
+    dgu = torch.zeros(off + gu.size, device=G.DEV)
+    dgu[off:] = G.dev(gu).reshape(-1)
+    h = torch.zeros(off + P * ffs + 1, dtype=torch.int16, device=G.DEV)
+    L.call("fnx_swiglu_h16", dgu[off:].data_ptr(), ffs, P, h[off:].data_ptr(), L.stream())
+    G.sync()
+    got = G.host(h, np.uint16)
+    assert np.array_equal(got[off:off + P * ffs].reshape(P, ffs), O.swiglu_h16(gu, ffs))
+    assert not got[:off].any() and got[-1] == 0

@@ -479,7 +479,7 @@ def test_commits_neither_wait_nor_keep_the_table():
 
     from sfnx_b200.window import LaneSet, StackShape, SyntheticStack, WindowRunner
 
-    shape = StackShape(n=512, nexp=32, topk=4, ff=128, nkh=2, nvh=4, nq=8, nkv=2, hd=256, nrot=64, vocab=512, kinds=[0, 1, 0], ctx=600, kv_slack=64)
+    shape = StackShape(n=512, nexp=32, topk=4, ff=256, nkh=2, nvh=4, nq=8, nkv=2, hd=256, nrot=64, vocab=512, kinds=[0, 1, 0], ctx=600, kv_slack=64)
     stack = SyntheticStack(shape, seed=21, device="cuda:0", gdn_log=False)
     lanes = LaneSet(stack, 2, 3)
     runner = WindowRunner(stack, 6, lanes=lanes)
@@ -510,3 +510,53 @@ def test_commits_neither_wait_nor_keep_the_table():
     assert waiting, "commit_lanes waited for the GPU"
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("nseg", [0, 2])
+def test_launched_windows_equal_called_ones(nseg):
+    """The three ways a window is enqueued give the same bits: the call from the host (its graph uploads and reads back), launch()
+    between an upload and a read-back of the caller's, and no graph at all; a sampled window of one sequence, and one of two."""
+    import torch
+
+    from sfnx_b200.window import LaneSet, StackShape, SyntheticStack, WindowRunner
+
+    shape = StackShape(n=512, nexp=32, topk=4, ff=256, nkh=2, nvh=4, nq=8, nkv=2, hd=256, nrot=64, vocab=512, kinds=[0, 1, 0], ctx=600, kv_slack=64)
+    stack = SyntheticStack(shape, seed=23, device="cuda:0", gdn_log=not nseg)
+    lanes = LaneSet(stack, nseg, 3) if nseg else None
+    T = 3 * nseg or 5
+    kw = {"lanes": lanes} if nseg else {"sampled": True}
+    rng = np.random.default_rng(24)
+    ids = [int(v) for v in rng.integers(0, shape.vocab, T)]
+    states = [t for l in sorted(lanes.S) for t in lanes.S[l] + lanes.hist[l]] if nseg else [t for pair in stack.gdn_state for t in pair]
+    before = [t.clone() for t in states]
+
+    runners = {g: WindowRunner(stack, T, graph=g, **kw) for g in (False, True)}   # (building one runs windows at position 0)
+
+    def run(graph, called):
+        r = runners[graph]
+        for t, b in zip(states, before):
+            t.copy_(b)
+        torch.cuda.synchronize()
+        if called:
+            best = r.window_lanes(ids, [40, 90], [1, 2]) if nseg else r.window(ids, 600, 1)
+        else:
+            r.h_in_np[:T] = ids
+            r.h_in_np[-2:] = 600, 1
+            with torch.cuda.stream(r.stream):
+                if nseg:
+                    lanes.positions([40, 90], [1, 2])
+                r.d_in.copy_(r.h_in)
+                r.launch()
+            r.stream.synchronize()
+            best = r.all_i[0].tolist()
+        torch.cuda.synchronize()
+        assert int(r.err[0]) == 0
+        out = [r.logits.clone()] + [t.clone() for t in states] + ([r.h_cv.cuda() if called else r.all_cv.clone()] if not nseg else [])
+        return best, out
+
+    want, ref = run(False, True)
+    for graph, called in ((True, True), (True, False)):
+        best, got = run(graph, called)
+        assert list(best) == list(want)
+        for a, b in zip(got, ref):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32)), (graph, called)
