@@ -70,11 +70,7 @@ __global__ void k_hc_add_streams(const float* __restrict__ h, const float* __res
 __device__ __forceinline__ float hc_gate(const HcArgs& a, int t, int c) {
     return fmul(2.0f, ex_sigmoid(fdiv(a.inj_prev[t * a.hc + c], (float) a.hc)));
 }
-// integer dots are started at the bits of 1.5 * 2^23: as floats minus that, (float) dot, without a convert instruction
-// (a quarter of the rate of the multiply-adds; the dots stay under 2^22)
-constexpr int HC_MAGIC = 0x4B400000;
-__device__ __forceinline__ float hc_float(int dot) { return fsub(__int_as_float(dot), 12582912.0f); }
-__device__ __forceinline__ int hc_dot8(const uint2 w, const int2 x) { return __dp4a((int) w.y, x.y, __dp4a((int) w.x, x.x, HC_MAGIC)); }
+__device__ __forceinline__ int hc_dot8(const uint2 w, const int2 x) { return __dp4a((int) w.y, x.y, __dp4a((int) w.x, x.x, 0)); }
 // rs of row k, stream c from the slices' square sums, the slices in ascending order
 __device__ __forceinline__ float hc_rs(const HcArgs& a, int k, int c) {
     const int ns = a.n * a.hc / HC_SL, sps = a.n / HC_SL;
@@ -182,7 +178,7 @@ __global__ void __launch_bounds__(HC_DT) k_hc_down(const HcArgs a) {
             for (int q = 0; q < NQ; ++q) {
                 const int ch = q * HC_TPR + j;
                 acc = ffma(fmul(__uint_as_float(wr[2 * NQ + q]), xd[k * (HC_SL / 32) + ch / 4]),
-                           hc_float(hc_dot8(make_uint2(wr[2 * q], wr[2 * q + 1]), *reinterpret_cast<const int2*>(xq + (size_t) k * HC_SL + ch * 8))), acc);
+                           (float) hc_dot8(make_uint2(wr[2 * q], wr[2 * q + 1]), *reinterpret_cast<const int2*>(xq + (size_t) k * HC_SL + ch * 8)), acc);
             }
         } else {
 #pragma unroll
@@ -306,7 +302,7 @@ __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
         for (int cc = 0; cc < HC_MAXS; ++cc) {
             if (cc >= hc) break;
             const uint4 w0 = wq[cc][0], w1 = wq[cc][1];
-            int sacc = __dp4a((int) w0.x, x0.x, HC_MAGIC);
+            int sacc = __dp4a((int) w0.x, x0.x, 0);
             sacc = __dp4a((int) w0.y, x0.y, sacc);
             sacc = __dp4a((int) w0.z, x0.z, sacc);
             sacc = __dp4a((int) w0.w, x0.w, sacc);
@@ -314,7 +310,7 @@ __global__ void __launch_bounds__(HC_UT) k_hc_up(const HcArgs a) {
             sacc = __dp4a((int) w1.y, x1.y, sacc);
             sacc = __dp4a((int) w1.z, x1.z, sacc);
             sacc = __dp4a((int) w1.w, x1.w, sacc);
-            float acc = fmul(fmul(wsc[cc], dl), hc_float(sacc));   // an idle lane: 0 * dl * 0
+            float acc = fmul(fmul(wsc[cc], dl), (float) sacc);   // an idle lane: 0 * dl * 0
             for (int o = 1; o < HC_TPU; o <<= 1) acc = fadd(acc, __shfl_xor_sync(0xffffffffu, acc, o));
             if (uj == 0) gs[((size_t) k * hc + cc) * HC_UPC + udd] = acc;
         }
