@@ -782,7 +782,10 @@ static int attn_partial_rows(const float* qg, const uint16_t* kc, const uint16_t
         return 0;
     };
     // rows with a list of their own go in a launch of their own.  Wide slices when the rows are one sequence's and make
-    // more than a narrow one; narrow ones for rows of several sequences, whose groups are small
+    // more than a narrow one; narrow ones for rows of several sequences, whose groups are small.  Narrow against wide, us, 24 / 4
+    // heads of 256, sequences x rows over f16 positions: 6 x 2 over 14 336 259 / 619, 8 x 2 over 8192 253 / 519, 5 x 3 278 / 389,
+    // 4 x 4 244 / 281, 3 x 5 255 / 299; but 2 x 8, whose groups fill a wide slice, 239 / 181 (305 / 200 over int8 rows, 1042 / 639
+    // over 40 000 positions): how many rows a sequence has is known on the device only
     const bool few = qpk <= 8, wide = !lr.pos && T * qpk > 12;
     if (hd == 256) {
         if (wide ? AX_RUN(256, 48, cells ? 1 : 0) : AX_RUN(256, 12, cells ? 1 : 0)) return 1;

@@ -5,15 +5,15 @@
 //
 // A block's integer dot of 128 weight rows against the window's 16 rows is ONE tcgen05.mma (kind::i8, M 128, N 16, K 32)
 // into 16 columns of tensor memory; nothing is accumulated on the tensor cores, because every block has scales of its own.
-// A persistent CTA (one per SM) walks 128-row tiles:
-//   warp 16   the TMA unit's driver: for every 128 bytes of K (four blocks) one cp.async.bulk.tensor load of the 128 x 128
-//             byte weight tile into a 128-byte-swizzled stage (six stages), and per tile one load of its f16 block scales;
-//             it starts before the kernel ahead in the stream has finished (weights depend on nothing in the window)
+// A persistent CTA (one per SM) walks tiles of H rows, 64 to 128 (q8s_umma_launch says which):
+//   warp 16   the TMA unit's driver: for every 128 bytes of K (four blocks) one cp.async.bulk.tensor load of the tile's H x 128
+//             bytes into a 128-byte-swizzled stage (six stages; the MMAs read 128 rows, those past H make rows of the result
+//             that nobody reads), and per tile its f16 block scales in boxes of 16 columns; it starts before the kernel ahead in the stream has finished (weights depend on nothing in the window)
 //   warp 17   issues the four MMAs of a stage, each into its own 16 columns of one of four 128-column groups of tensor
 //             memory; tcgen05.commit hands the stage back to the TMA warp and, every second stage, the group to the epilogue
 //   warps 0-15  the epilogue: warp w reads rows 32 (w % 4) .. + 31 (its quarter of tensor memory) and window rows
-//             4 (w / 4) .. + 3 (the warps of rows that the window does not have leave at once): tcgen05.ld, the integer dots to float by the 1.5 * 2^23 offset (no convert instruction),
-//             scale by fl(dw da) and add - sixteen warps so that the CUDA-core work of a 4 KB block step (128 rows x 16
+//             4 (w / 4) .. + 3 (the warps of rows that the window does not have leave at once): tcgen05.ld, the integer dots to
+//             float by the 1.5 * 2^23 offset (no convert instruction), scale by fl(dw da) and add - sixteen warps so that the CUDA-core work of a 4 KB block step (128 rows x 16
 //             values) stays well under the time HBM needs to deliver the step.
 // The window's activations (int8 plane as the MMAs' B operand, 16 rows x K, and their float scales) are staged once per
 // CTA.  Every wait is bounded; a wait that runs out sets bit 8 of the fault word and the CTA finishes without waiting again.

@@ -778,7 +778,7 @@ int fnx_moe_gate_up(const FnxExperts* A, const FnxJob* jobs, const int* njobs, i
         // blocks of 128 rows with direct 16-byte loads one step ahead (measured faster than staging the weights through
         // shared memory, by cp.async rings or bulk copies: there every operand crosses the shared-memory pipe)
         // rows of 128 a block, of 64 where an expert has few rows or a window so few jobs that the longer blocks would not
-        // give every multiprocessor one: the launch is over sooner (one row's ten jobs at 1536 x 3072: 12.0 us, now 9.6)
+        // give every multiprocessor (148) one: the launch is over sooner (one row's ten jobs at 1536 x 3072: 12.0 us, now 9.6)
         const int blocks128 = (nrows + GU_THREADS / 2 - 1) / (GU_THREADS / 2) * njobs_max;
         const int R = (nrows <= 512 || blocks128 < 148) && (n / 512) % 2 == 0 ? 2 : 4, rpb = GU_THREADS / 8 * R;   // the step count must stay even
         const dim3 grid((nrows + rpb - 1) / rpb, njobs_max);
