@@ -461,7 +461,7 @@ def main():
                    "numerator": "accepted tokens per step, mean over all timed steps" + ("" if sampled else " (= 1 + leading true Bernoulli draws: %s)" %
                                                                                           ("checked" if draws_agree else "NOT reproduced by the windows"))},
         "e2e": {"value": round(accepted_per_step / (e2e_ms / args.steps * 1e-3), 2), "unit": "tok/s", "ms_per_step": round(e2e_ms / args.steps, 4),
-                "h2d_bytes_per_step": nseq * (runners[0].h2d_bytes + runners[0].job_bytes),
+                "h2d_bytes_per_step": nseq * runners[0].h2d_bytes,   # (the rollback's tables are launch parameters)
                 "d2h_bytes_per_step": nseq * (runners[0].d2h_bytes + (world * T * 64 * 8 if sampled else 0)),
                 "accepted_per_step": round(e2e_accepted / (args.steps * repeats), 3)},
         "gpu_launches": int(kernels_per_window * nseq * args.steps), "kernels_per_window": int(kernels_per_window),
