@@ -22,8 +22,8 @@
 // What bounds it: the producers' dequantisation and the shared-memory pipe (its stores and the weights' 16-byte loads), not
 // the tensor cores or HBM.  256 rows a tile halve the copies of activation rows (against 128 rows and two CTAs an SM), and
 // running on from tile to tile hides a tile's start and end.  4096 tokens (1010 jobs, 512 experts
-// of 1536 x 3072 and 3072 x 768): gate|up Q4_K 1.18 -> 0.87 ms, down Q6_K 0.95 -> 0.69; Q8_0 1.42 -> 0.91 and 0.92 -> 0.58;
-// 130 tokens, Q4_K/Q6_K: 0.92 -> 0.60 and 0.64 -> 0.53.
+// of 1536 x 3072 and 3072 x 768): gate|up Q4_K 1.18 -> 0.82 ms, down Q6_K 0.95 -> 0.63; Q8_0 1.42 -> 0.90 and 0.92 -> 0.51;
+// 130 tokens, Q4_K/Q6_K: 0.92 -> 0.51 and 0.64 -> 0.46.
 #include <algorithm>
 
 #include "common.cuh"
