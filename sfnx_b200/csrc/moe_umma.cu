@@ -15,7 +15,7 @@
 //                swizzle) in one of three shared-memory stages.  A tile's result is written out after the next
 //                tile's first stages are full, so the tensor cores and the copies never wait for it.
 //   warp 16      issues a full stage's MMAs (K 16 each) and lets tcgen05.commit hand the stage back
-//   warp 17      asks for the raw weights (TMA tensor loads into a ring of their own)
+//   warp 17      copies the raw weights (asynchronous copies into a ring of their own)
 //   warps 18-23  the jobs' activation rows (the B operand, same form) by asynchronous copies, two warps a stage
 // Every wait is bounded and feeds the device fault word.
 //
@@ -65,12 +65,14 @@ struct MuArgs {
     unsigned* fault;
 };
 
-// The raw weights of a tile: the plane that holds nearly all of them comes through a ring in shared memory by TMA tensor
-// loads, STEPS steps (64 columns each) of the tile's 256 rows a load: Q4_K whole super-blocks (144 bytes a row, four steps;
-// rows 144 bytes apart are conflict-free as they are), Q8_0 the quants (64 bytes, swizzled), Q6_K the low nibbles (32
-// bytes, swizzled).  What is left (scales, Q6_K's high bits) a thread loads for its own row and half, a step ahead.
-// (Every thread loading its own row's pieces put 16 lines into each request and was the slowest part: 0.7 ms of 1.2 for
-// gate|up of 512 experts of 1536 x 3072 with everything else taken out.)
+// The raw weights of a tile: the plane that holds nearly all of them comes through a ring in shared memory, STEPS steps (64
+// columns each) of the tile's 256 rows a load, in 16-byte pieces by asynchronous copies of one warp, whose lanes take
+// neighbouring pieces: Q4_K whole super-blocks (144 bytes a row, four steps; rows 144 bytes apart are conflict-free as they
+// are), Q8_0 the quants (64 bytes, swizzled), Q6_K the low nibbles (32 bytes, swizzled).  What is left (scales, Q6_K's high
+// bits) a thread loads for its own row and half, a step ahead.  (Every thread loading its own row's pieces put 16 lines
+// into each request and was the slowest part: 0.7 ms of 1.2 for gate|up of 512 experts of 1536 x 3072 with everything else
+// taken out.  TMA tensor loads do not fit: the host does not know how many experts there are, and a tensor map that claims
+// more of them than are in memory may not be given to the unit; it faulted where memory ends soon after a small matrix.)
 // volatile: the loads stay where they are written, a step ahead of their use
 __device__ __forceinline__ uint2 mu_ld8(const void* p) {
     uint2 v;
@@ -84,6 +86,9 @@ __device__ __forceinline__ unsigned mu_ld2(const void* p) {
 }
 template <int TYPE> struct MuRaw {   // Q8_0, Q6_K
     static constexpr int STEPS = 1, WIDTH = TYPE == FNX_Q8_0 ? 64 : 32, SLOTS = 4;
+    static __device__ __forceinline__ int row_bytes(const MuArgs& a) { return TYPE == FNX_Q8_0 ? a.ncols : a.ncols / 2; }
+    static __device__ __forceinline__ size_t expert_bytes(const MuArgs& a) { return TYPE == FNX_Q8_0 ? a.stride : a.stride * 16; }
+    static __device__ __forceinline__ int swizzle(int row) { return TYPE == FNX_Q8_0 ? (row >> 1) & 3 : (row >> 2) & 1; }   // of a row's pieces
     uint4 q0, q1;   // Q8_0: the 32 quants; Q6_K: q0 = low nibbles, q1.xy = high bits
     unsigned s, d;  // Q8_0: s = scale; Q6_K: s = the two scales, d = d
     __device__ __forceinline__ void fetch(const MuArgs& a, int expert, int row, int half, int step) {
@@ -100,18 +105,20 @@ template <int TYPE> struct MuRaw {   // Q8_0, Q6_K
         }
     }
     __device__ __forceinline__ void begin(const unsigned char*, int) {}
-    __device__ __forceinline__ void read(const unsigned char* slot, int row, int half, int) {   // the swizzles of 64 and 32 bytes
+    __device__ __forceinline__ void read(const unsigned char* slot, int row, int half, int) {
         if (TYPE == FNX_Q8_0) {
             const uint4* r = reinterpret_cast<const uint4*>(slot + row * 64);
-            const int sw = (row >> 1) & 3;
-            q0 = r[(2 * half) ^ sw], q1 = r[(2 * half + 1) ^ sw];
+            q0 = r[(2 * half) ^ swizzle(row)], q1 = r[(2 * half + 1) ^ swizzle(row)];
         } else {
-            q0 = reinterpret_cast<const uint4*>(slot + row * 32)[half ^ ((row >> 2) & 1)];
+            q0 = reinterpret_cast<const uint4*>(slot + row * 32)[half ^ swizzle(row)];
         }
     }
 };
 template <> struct MuRaw<FNX_Q4_K> {
     static constexpr int STEPS = 4, WIDTH = 144, SLOTS = 2;
+    static __device__ __forceinline__ int row_bytes(const MuArgs& a) { return a.ncols / 256 * 144; }
+    static __device__ __forceinline__ size_t expert_bytes(const MuArgs& a) { return a.stride; }
+    static __device__ __forceinline__ int swizzle(int) { return 0; }
     uint4 hd, q[4];
     __device__ __forceinline__ void fetch(const MuArgs&, int, int, int, int) {}
     __device__ __forceinline__ void begin(const unsigned char* slot, int row) { hd = *reinterpret_cast<const uint4*>(slot + row * 144); }
@@ -242,7 +249,7 @@ __device__ int mu_list_pairs(const FnxBigJob* jobs, int base, int cnt, int& run,
 
 // out[jb.out[j] * nrows + row] = sum_k W_e[row][k] x[jb.y[j] * ncols + k]
 template <int TYPE>
-__global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, const __grid_constant__ CUtensorMap wmap) {
+__global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a) {
     using Raw = MuRaw<TYPE>;
     const int tid = threadIdx.x, warp = (int) um_uniform(tid >> 5), lane = tid & 31;
     const int njobs = min(*a.njobs, a.njobs_cap);
@@ -262,7 +269,7 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&empty[s])));
         }
         for (int s = 0; s < Raw::SLOTS; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_s32(&rfull[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(um_s32(&rfull[s])));   // the loader's lanes
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(um_s32(&rempty[s])), "r"(MU_PROD / 32));
         }
         for (int s = 0; s < 2; ++s) {
@@ -376,20 +383,32 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a, cons
             }
             if (prev >= 0) write_out(prev, seq - 1);
         } else if (warp == MU_PROD / 32 + 1) {
-            // ---- the raw weights' loads, as far ahead as the ring holds, across the ends of tiles
-            if (lane == 0) {
-                const auto landed = [&](unsigned s, unsigned parity) { return um_wait(&rfull[s], parity, a.fault); };
-                const auto used = [&](unsigned s, unsigned parity) { return um_wait(&rempty[s], parity, a.fault); };
-                for (int it = first; it < items && ring.alive; it += stride) {
-                    const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
-                    for (int c = 0; c < nsteps && ring.acquire(used, landed); ++c) {
-                        const unsigned slot = ring.slot;
-                        um_expect_tx(&rfull[slot], Raw::WIDTH * MU_BM);
-                        um_tma3d(um_s32(raw + slot * (Raw::WIDTH * MU_BM)), &wmap, c * Raw::WIDTH, it % ntiles * MU_BM, expert, &rfull[slot]);
-                        ring.asked();
+            // ---- the raw weights' copies, as far ahead as the ring holds, across the ends of tiles.  Rows past the matrix repeat
+            // the last one, pieces past a row's end are left out: nothing is read that is not the matrix's
+            const auto landed = [&](unsigned s, unsigned parity) { return um_wait(&rfull[s], parity, a.fault); };
+            const auto used = [&](unsigned s, unsigned parity) { return um_wait(&rempty[s], parity, a.fault); };
+            constexpr int PC = Raw::WIDTH / 16;   // pieces a row
+            const int row_bytes = Raw::row_bytes(a);
+            for (int it = first; it < items && ring.alive; it += stride) {
+                const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
+                const unsigned char* src = a.a + (size_t) expert * Raw::expert_bytes(a);
+                const int row0 = it % ntiles * MU_BM, last = a.nrows - 1 - row0;
+                src += (size_t) row0 * row_bytes;
+                for (int c = 0; c < nsteps; ++c) {
+                    ring.alive = __all_sync(0xffffffffu, ring.acquire(used, landed));
+                    if (!ring.alive) break;
+                    const unsigned dst = um_s32(raw + ring.slot * (Raw::WIDTH * MU_BM));
+                    const int at = c * Raw::WIDTH;
+#pragma unroll 8
+                    for (int e = lane; e < MU_BM * PC; e += 32) {
+                        const int row = e / PC, pc = e % PC;
+                        if (at + 16 * pc < row_bytes)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + row * Raw::WIDTH + ((pc ^ Raw::swizzle(row)) << 4)),
+                                         "l"(src + (size_t) (unsigned) (min(row, last) * row_bytes + at + 16 * pc)));
                     }
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(um_s32(&rfull[ring.slot])) : "memory");
+                    ring.asked();
                 }
-                ring.drain(landed);   // no load is in flight when the block ends
             }
         } else if (warp > MU_PROD / 32) {
             // ---- the activation rows, by asynchronous copies, two warps a step in turn: every stage's copies are issued side by side.  Lane i takes
@@ -509,33 +528,20 @@ static int moe_umma(const char* what, const FnxExperts* A, const FnxBigJob* jobs
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return fail("%s: no device", what);
     const int grid = (int) std::min<long long>(nsm, (long long) ((A->nrows + MU_BM - 1) / MU_BM) * njobs_cap);
-    // the raw weights' plane as bytes (column, row, expert); how many experts there are is the jobs' business
-    CUtensorMap wmap;
-    const UmEncode encode = um_encoder();
-    FNX_REQUIRE(encode, "%s: the driver has no tensor-map encoder", what);
-    const auto map = [&](int row_bytes, size_t expert_bytes, int width, CUtensorMapSwizzle swizzle) {
-        const cuuint64_t dims[3] = {(cuuint64_t) row_bytes, (cuuint64_t) A->nrows, 1u << 20}, strides[2] = {(cuuint64_t) row_bytes, (cuuint64_t) (expert_bytes ? expert_bytes : row_bytes)};
-        const cuuint32_t box[3] = {(cuuint32_t) width, MU_BM, 1}, ones[3] = {1, 1, 1};
-        return encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(A->a), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    };
 #define MU_LAUNCH(T)                                                            \
     if (smem_optin(k_moe_umma<T>, MU_SMEM, what)) return 1;                     \
-    k_moe_umma<T><<<grid, MU_THREADS, MU_SMEM, st>>>(a, wmap);                        \
+    k_moe_umma<T><<<grid, MU_THREADS, MU_SMEM, st>>>(a);                        \
     return launch_ok(what);
     if (A->type == FNX_Q4_K) {
         FNX_REQUIRE(A->ncols % 256 == 0 && ((uintptr_t) A->a % 16) == 0 && A->stride % 16 == 0, "%s q4_K: %d columns, rows 16-byte aligned", what, A->ncols);
-        FNX_REQUIRE(map(A->ncols / 256 * 144, A->stride, 144, CU_TENSOR_MAP_SWIZZLE_NONE), "%s q4_K: tensor map", what);
         MU_LAUNCH(FNX_Q4_K)
     }
     if (A->type == FNX_Q8_0) {
         FNX_REQUIRE(((uintptr_t) A->a % 16) == 0 && A->stride % 16 == 0 && A->stride_b % 2 == 0, "%s q8_0: planes 16-byte aligned", what);
-        FNX_REQUIRE(map(A->ncols, A->stride, 64, CU_TENSOR_MAP_SWIZZLE_64B), "%s q8_0: tensor map", what);
         MU_LAUNCH(FNX_Q8_0)
     }
     if (A->type == FNX_Q6_K) {
         FNX_REQUIRE(((uintptr_t) A->a % 16) == 0 && ((uintptr_t) A->b % 8) == 0, "%s q6_K: unit planes not aligned", what);
-        FNX_REQUIRE(map(A->ncols / 2, A->stride * 16, 32, CU_TENSOR_MAP_SWIZZLE_32B), "%s q6_K: tensor map", what);
         MU_LAUNCH(FNX_Q6_K)
     }
 #undef MU_LAUNCH

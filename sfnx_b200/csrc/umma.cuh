@@ -65,11 +65,6 @@ __device__ __forceinline__ void um_tma2d(unsigned dst, const CUtensorMap* map, i
                  "r"(x), "r"(y), "r"(um_s32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void um_tma3d(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(map),
-                 "r"(x), "r"(y), "r"(z), "r"(um_s32(bar))
-                 : "memory");
-}
 // a contiguous run of bytes (both addresses and the size multiples of 16)
 __device__ __forceinline__ void um_bulk(unsigned dst, const void* src, unsigned bytes, unsigned long long* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),

@@ -223,3 +223,54 @@ def test_swiglu_of_any_width_and_address(P, ffs, off):
     got = G.host(h, np.uint16)
     assert np.array_equal(got[off:off + P * ffs].reshape(P, ffs), O.swiglu_h16(gu, ffs))
     assert not got[:off].any() and got[-1] == 0
+
+
+@pytest.mark.parametrize("kind,rows,cols", [("q8_0", 100, 32), ("q8_0", 100, 96), ("q8_0", 300, 64), ("q8_0", 1, 32), ("q4k", 100, 256), ("q4k", 64, 512),
+                                            ("q6p", 256, 32), ("q6p", 512, 96)])
+def test_nothing_is_read_past_the_end_of_memory(kind, rows, cols):
+    """Small matrices, jobs and activation rows that end where their mapped memory does: buffers of 12 MB, mappings of their
+    own, each with its array in the last bytes."""
+    import torch
+
+    from oracle import binding as O
+    from sfnx_b200 import lib as L
+    from tests import gpu_util as G
+
+    nexp, rng = 4, np.random.default_rng(rows + cols)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    keep = []
+
+    def tail(a):   # the array's bytes at the end of a mapping, on a 16-byte boundary (what is left over lies behind it)
+        b = np.ascontiguousarray(a).view(np.uint8).reshape(-1)
+        buf = torch.zeros(12 << 20, dtype=torch.uint8, device=G.DEV)
+        at = (buf.numel() - b.size) // 16 * 16
+        buf[at:at + b.size] = torch.from_numpy(b.copy()).to(G.DEV)
+        keep.append(buf)
+        return buf.data_ptr() + at
+
+    if kind == "q8_0":
+        q = rng.integers(-127, 128, (nexp, rows, cols)).astype(np.int8)
+        d = (0.01 * rng.random((nexp, rows, cols // 32)) + 1e-3).astype(np.float16).view(np.uint16)
+        ex, w16 = L.Experts(L.Q8_0, rows, cols, tail(q), tail(d), None, None, rows * cols, rows * (cols // 32) * 2), O.mma_weights_q8(q, d)
+    elif kind == "q4k":
+        w = cases.moe_weights(n=cols, nexp=nexp, ffs=32 * ((rows // 2 + 31) // 32), seed=46)
+        blocks = np.ascontiguousarray(w["gu_q4k"].reshape(nexp, -1)[:, :rows * (cols // 256) * 144])
+        ex, w16 = L.Experts(L.Q4_K, rows, cols, tail(blocks), None, None, None, blocks.shape[1], 0), O.mma_weights_q4k(blocks, nexp * rows, cols)
+    else:
+        planes = cases.moe_weights(n=rows, nexp=nexp, ffs=cols, seed=46)["dn_planes"]
+        ex, w16 = L.Experts(L.Q6_K, rows, cols, *[tail(p) for p in planes], rows * (cols // 32), 0), O.mma_weights_q6p(planes, nexp * rows, cols)
+    n = np.array([1, 40, 64, 3, 64, 17])
+    jobs = np.zeros(len(n), O.BIGJOB_DTYPE)
+    jobs["w"], jobs["n"] = [0, 1, 2, 2, 3, 3], n
+    for j, at in enumerate(np.cumsum(n) - n):
+        jobs[j]["y"][:n[j]], jobs[j]["out"][:n[j]] = (np.arange(n[j]) + at) % 71, np.arange(n[j]) + at
+    P = int(n.sum())
+    x16 = _f16_bits(rng.standard_normal((71, cols)))
+    out = torch.full((P, rows), float("nan"), device=G.DEV)
+    nj = G.dev(np.array([len(n), 0], np.int32))
+    L.call("fnx_moe_gate_up_mma", C.byref(ex), tail(jobs), nj.data_ptr(), len(n), tail(x16), out.data_ptr(), L.stream())
+    G.sync()
+    assert L.load().fnx_device_fault() == 0
+    ref, mag = O.moe_mma(w16, jobs, len(jobs), x16, rows, P)
+    _close(G.host(out), ref, mag, cols)
