@@ -66,9 +66,10 @@ struct MuArgs {
 };
 
 // The raw weights of a tile: the plane that holds nearly all of them comes through a ring in shared memory, STEPS steps (64
-// columns each) of the tile's 256 rows a load, in 16-byte pieces by asynchronous copies of one warp, whose lanes take
-// neighbouring pieces: Q4_K whole super-blocks (144 bytes a row, four steps; rows 144 bytes apart are conflict-free as they
-// are), Q8_0 the quants (64 bytes, swizzled), Q6_K the low nibbles (32 bytes, swizzled).  What is left (scales, Q6_K's high
+// columns each) of the tile's 256 rows a load, copied by one warp in 16-byte asynchronous copies, neighbouring pieces by neighbouring
+// lanes: Q4_K whole super-blocks (144 bytes a row, four steps; rows 144 bytes apart are conflict-free as they are), Q8_0 the
+// quants (64 bytes, swizzled), Q6_K the low nibbles (32 bytes, swizzled).  A bulk copy a row instead took gate|up of 4096 tokens
+// from 0.87 to 2.08 ms.  What is left (scales, Q6_K's high
 // bits) a thread loads for its own row and half, a step ahead.  (Every thread loading its own row's pieces put 16 lines
 // into each request and was the slowest part: 0.7 ms of 1.2 for gate|up of 512 experts of 1536 x 3072 with everything else
 // taken out.  TMA tensor loads do not fit: the host does not know how many experts there are, and a tensor map that claims
@@ -387,8 +388,12 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a) {
             // the last one, pieces past a row's end are left out: nothing is read that is not the matrix's
             const auto landed = [&](unsigned s, unsigned parity) { return um_wait(&rfull[s], parity, a.fault); };
             const auto used = [&](unsigned s, unsigned parity) { return um_wait(&rempty[s], parity, a.fault); };
-            constexpr int PC = Raw::WIDTH / 16;   // pieces a row
             const int row_bytes = Raw::row_bytes(a);
+            unsigned off[9];   // Q4_K: this lane's pieces among 32 rows
+            if (TYPE == FNX_Q4_K) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) off[k] = (unsigned) ((lane + 32 * k) / 9 * row_bytes + (lane + 32 * k) % 9 * 16);
+            }
             for (int it = first; it < items && ring.alive; it += stride) {
                 const int expert = a.stride ? a.jobs[job_of(it)].w : 0;   // stride 0: one matrix for all
                 const unsigned char* src = a.a + (size_t) expert * Raw::expert_bytes(a);
@@ -398,13 +403,42 @@ __global__ void __launch_bounds__(MU_THREADS, 1) k_moe_umma(const MuArgs a) {
                     ring.alive = __all_sync(0xffffffffu, ring.acquire(used, landed));
                     if (!ring.alive) break;
                     const unsigned dst = um_s32(raw + ring.slot * (Raw::WIDTH * MU_BM));
-                    const int at = c * Raw::WIDTH;
-#pragma unroll 8
-                    for (int e = lane; e < MU_BM * PC; e += 32) {
-                        const int row = e / PC, pc = e % PC;
-                        if (at + 16 * pc < row_bytes)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + row * Raw::WIDTH + ((pc ^ Raw::swizzle(row)) << 4)),
-                                         "l"(src + (size_t) (unsigned) (min(row, last) * row_bytes + at + 16 * pc)));
+                    const unsigned char* from = src + c * Raw::WIDTH;
+                    if constexpr (TYPE == FNX_Q4_K) {   // nine pieces a row, one after the other in the slot: 32 rows every nine pieces of a lane
+                        const unsigned to = dst + 16 * lane;
+                        if (last >= MU_BM - 1) {
+                            const unsigned char* q = from;
+#pragma unroll
+                            for (int b = 0; b < MU_BM / 32; ++b, q += 32 * row_bytes)
+#pragma unroll
+                                for (int k = 0; k < 9; ++k)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (9 * b + k) * 512), "l"(q + off[k]));
+                        } else {
+#pragma unroll 4
+                            for (int i = 0; i < MU_BM * 9 / 32; ++i) {
+                                const int e = lane + 32 * i;
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 512 * i),
+                                             "l"(from + (size_t) (unsigned) (min(e / 9, last) * row_bytes + 16 * (e % 9))));
+                            }
+                        }
+                    } else {   // a lane the same piece of every 32 / PC-th row (the swizzle is the same for all of them)
+                        constexpr int PC = Raw::WIDTH / 16, RP = 32 / PC;
+                        const int r0 = lane / PC, pc = lane % PC;
+                        const unsigned to = dst + r0 * Raw::WIDTH + ((pc ^ Raw::swizzle(r0)) << 4);
+                        if (c * Raw::WIDTH + 16 * pc < row_bytes) {
+                            if (last >= MU_BM - 1) {
+                                const unsigned char* q = from + r0 * row_bytes + 16 * pc;
+                                const int step = RP * row_bytes;
+#pragma unroll
+                                for (int i = 0; i < MU_BM / RP; ++i, q += step)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * RP * Raw::WIDTH), "l"(q));
+                            } else {
+#pragma unroll 4
+                                for (int i = 0; i < MU_BM / RP; ++i)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * RP * Raw::WIDTH),
+                                                 "l"(from + (size_t) (unsigned) (min(r0 + RP * i, last) * row_bytes + 16 * pc)));
+                            }
+                        }
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(um_s32(&rfull[ring.slot])) : "memory");
                     ring.asked();
