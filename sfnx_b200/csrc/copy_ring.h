@@ -1,4 +1,4 @@
-// The bookkeeping of a ring of SLOTS shared-memory buffers that one thread fills by asynchronous copies (the TMA unit's):
+// The bookkeeping of a ring of SLOTS shared-memory buffers that one thread (or the lanes of a warp together) fills by asynchronous copies:
 // copy k goes into slot k % SLOTS and completes phase k / SLOTS of the slot's `full` barrier; its readers complete phase
 // k / SLOTS of the slot's `empty` barrier when they are done with it.  Plain C++, so that a test on the CPU can run it.
 //

@@ -22,8 +22,8 @@
 // What bounds it: the producers' dequantisation and the shared-memory pipe (its stores and the weights' 16-byte loads), not
 // the tensor cores or HBM.  256 rows a tile halve the copies of activation rows (against 128 rows and two CTAs an SM), and
 // running on from tile to tile hides a tile's start and end.  4096 tokens (1010 jobs, 512 experts
-// of 1536 x 3072 and 3072 x 768): gate|up Q4_K 1.18 -> 0.82 ms, down Q6_K 0.95 -> 0.63; Q8_0 1.42 -> 0.90 and 0.92 -> 0.51;
-// 130 tokens, Q4_K/Q6_K: 0.92 -> 0.51 and 0.64 -> 0.46.
+// of 1536 x 3072 and 3072 x 768): gate|up Q4_K 1.18 -> 0.84 ms, down Q6_K 0.95 -> 0.64; Q8_0 1.42 -> 0.89 and 0.92 -> 0.50;
+// 130 tokens, Q4_K/Q6_K: 0.92 -> 0.54 and 0.64 -> 0.48.
 #include <algorithm>
 
 #include "common.cuh"
@@ -66,14 +66,14 @@ struct MuArgs {
 };
 
 // The raw weights of a tile: the plane that holds nearly all of them comes through a ring in shared memory, STEPS steps (64
-// columns each) of the tile's 256 rows a load, copied by one warp in 16-byte asynchronous copies, neighbouring pieces by neighbouring
-// lanes: Q4_K whole super-blocks (144 bytes a row, four steps; rows 144 bytes apart are conflict-free as they are), Q8_0 the
-// quants (64 bytes, swizzled), Q6_K the low nibbles (32 bytes, swizzled).  A bulk copy a row instead took gate|up of 4096 tokens
-// from 0.87 to 2.08 ms.  What is left (scales, Q6_K's high
-// bits) a thread loads for its own row and half, a step ahead.  (Every thread loading its own row's pieces put 16 lines
-// into each request and was the slowest part: 0.7 ms of 1.2 for gate|up of 512 experts of 1536 x 3072 with everything else
-// taken out.  TMA tensor loads do not fit: the host does not know how many experts there are, and a tensor map that claims
-// more of them than are in memory may not be given to the unit; it faulted where memory ends soon after a small matrix.)
+// columns each) of the tile's 256 rows a load, copied by one warp in 16-byte asynchronous copies, neighbouring pieces by
+// neighbouring lanes: Q4_K whole super-blocks (144 bytes a row, four steps; rows 144 bytes apart are conflict-free as they
+// are), Q8_0 the quants (64 bytes, swizzled), Q6_K the low nibbles (32 bytes, swizzled).  A bulk copy a row instead took
+// gate|up of 4096 tokens from 0.87 to 2.08 ms.  What is left (scales, Q6_K's high bits) a thread loads for its own row and
+// half, a step ahead.  (Every thread loading its own row's pieces put 16 lines into each request and was the slowest part:
+// 0.7 ms of 1.2 for gate|up of 512 experts of 1536 x 3072 with everything else taken out.  TMA tensor loads do not fit: the
+// host does not know how many experts there are, and a tensor map that claims more of them than are in memory may not be
+// given to the unit; it faulted where memory ends soon after a small matrix.)
 // volatile: the loads stay where they are written, a step ahead of their use
 __device__ __forceinline__ uint2 mu_ld8(const void* p) {
     uint2 v;
